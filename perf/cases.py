@@ -401,8 +401,8 @@ def tolerance(case):
         return {"rel": 2e-15 if f64 else 1e-6}
     if call == "cg":
         return {"rel": 1e-14 if f64 else 3e-6}
-    if call == "bicgstab":  # its recurrences amplify a change in the order of a sum
-        return {"rel": 4e-12}
+    if call == "bicgstab":  # its recurrences amplify a change in the order of a sum, up to 9e-11 seen in 2D
+        return {"rel": 4e-10}
     if call == "gmres":
         return {"rel": 1e-14}
     # what the stopping residue leaves of the error on these operators
