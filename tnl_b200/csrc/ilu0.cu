@@ -6,9 +6,11 @@
 // scheduled by dependency levels: row i of L depends on the rows j < i it
 // references, row i of U on the rows j > i.  Levels are computed once on the
 // host (one pass over the pattern in row order), rows of a level run in
-// parallel, one kernel launch per level; the solves are captured once in a
-// CUDA graph and replayed; runs of small levels share one single-block
-// launch (a __syncthreads between levels).
+// parallel, one kernel launch per level.  The solves of factors with many
+// levels run as a pipeline of blocks, one launch per triangle
+// (ilu_pipe.cuh); those with few, wide levels as launches per level captured
+// once in a CUDA graph, runs of small levels sharing one single-block launch
+// (a __syncthreads between levels).
 //
 // Arithmetic per row follows ILU0.hpp:59-118 (IKJ order, L_ik = A_ik/U_kk,
 // then the updates of the rest of L_i and of U_i with U(k, j) looked up in
@@ -18,48 +20,13 @@
 #include <algorithm>
 #include <vector>
 
+#include "ilu_pipe.cuh"
 #include "internal.cuh"
+#include "reduce.cuh"
 #include "segview.cuh"
 
 namespace tnlb {
 namespace {
-
-template <typename Real>
-__device__ __forceinline__ Real mul_rn(Real a, Real b);
-template <>
-__device__ __forceinline__ double mul_rn<double>(double a, double b)
-{
-   return __dmul_rn(a, b);
-}
-template <>
-__device__ __forceinline__ float mul_rn<float>(float a, float b)
-{
-   return __fmul_rn(a, b);
-}
-template <typename Real>
-__device__ __forceinline__ Real sub_rn(Real a, Real b);
-template <>
-__device__ __forceinline__ double sub_rn<double>(double a, double b)
-{
-   return __dsub_rn(a, b);
-}
-template <>
-__device__ __forceinline__ float sub_rn<float>(float a, float b)
-{
-   return __fsub_rn(a, b);
-}
-template <typename Real>
-__device__ __forceinline__ Real div_rn(Real a, Real b);
-template <>
-__device__ __forceinline__ double div_rn<double>(double a, double b)
-{
-   return __ddiv_rn(a, b);
-}
-template <>
-__device__ __forceinline__ float div_rn<float>(float a, float b)
-{
-   return __fdiv_rn(a, b);
-}
 
 // One thread per row of the level.  lu holds A's values and is overwritten by
 // the factors; lstart/ustart/uend delimit the L and U parts of each row.
@@ -290,6 +257,133 @@ __global__ void __launch_bounds__(kIluPipeThreads)
    }
 }
 
+// One triangle's packed steps on the device.
+template <typename Real>
+struct PipeTri {
+   int32_t K = 0, npad = 0, parts = 0, consumers = 0;
+   PipeLayout lay{};
+   DeviceBuffer steps, part_step, rows_at, packed, ext;
+
+   template <bool Upper>
+   static const void* kernel(int k)
+   {
+      switch (k) {
+         case 1: return (const void*)k_ilu_pipe<Real, 1, Upper>;
+         case 2: return (const void*)k_ilu_pipe<Real, 2, Upper>;
+         case 3: return (const void*)k_ilu_pipe<Real, 3, Upper>;
+         case 4: return (const void*)k_ilu_pipe<Real, 4, Upper>;
+         default: return (const void*)k_ilu_pipe<Real, 8, Upper>;
+      }
+   }
+   template <bool Upper>
+   static int32_t row_size(int k)
+   {
+      switch (k) {
+         case 1: return PipeRow<Real, 1, Upper>::kBytes;
+         case 2: return PipeRow<Real, 2, Upper>::kBytes;
+         case 3: return PipeRow<Real, 3, Upper>::kBytes;
+         case 4: return PipeRow<Real, 4, Upper>::kBytes;
+         default: return PipeRow<Real, 8, Upper>::kBytes;
+      }
+   }
+   size_t smem() const { return (size_t)kPipeWindow * sizeof(Real) + (size_t)lay.stages * lay.stage_bytes; }
+
+   // progress[parts * 32] is followed, at the same place for both
+   // triangles, by the error word of the last (unused) part's slot.
+   template <bool Upper>
+   tnlb_status launch(const Real* in, Real* out, const Real* ext_src, int32_t* pr, cudaStream_t st) const
+   {
+      PipeArgs<Real> a{steps.as<PipeStep>(), part_step.as<int32_t>(), packed.as<unsigned char>(), in,
+                       ext.as<PipeExt>(), ext_src, out, pr, pr + kPipeMaxParts * 32, lay, consumers};
+      void* args[] = {&a};
+      TNLB_CUDA_TRY(cudaLaunchCooperativeKernel(kernel<Upper>(K), dim3(parts), dim3(32 * (consumers + 3 + lay.stages)),
+                                                args, smem(), st));
+      return TNLB_OK;
+   }
+
+   // The packed triangle of `plan`; beg/end delimit the entries of a row,
+   // `skip` of them not taken (U's pivot).  K stays 0 when a step has more
+   // external entries than a stage holds, or the plan is not worth it
+   // against `other_ns` of the level-by-level solve.
+   template <bool Upper>
+   tnlb_status build(PipePlan& plan, const PipeBuild& dev, int32_t k, const Real* lu, const int32_t* dst_of,
+                     double other_ns, cudaStream_t st)
+   {
+      const int32_t ns = (int32_t)plan.steps.size();
+      const int64_t n = (int64_t)plan.pos.size();
+      DeviceBuffer count;
+      TNLB_TRY_STATUS(count.alloc(sizeof(int32_t) * (size_t)ns));
+      TNLB_CUDA_TRY(cudaMemsetAsync(count.ptr, 0, sizeof(int32_t) * (size_t)ns, st));
+      k_pipe_count<<<grid_for(plan.npad, 256), 256, 0, st>>>(dev, count.as<int32_t>());
+      TNLB_CHECK_LAUNCH();
+      std::vector<int32_t> ec(ns);
+      TNLB_CUDA_TRY(cudaMemcpyAsync(ec.data(), count.ptr, sizeof(int32_t) * (size_t)ns, cudaMemcpyDeviceToHost, st));
+      TNLB_CUDA_TRY(cudaStreamSynchronize(st));
+      int64_t total = 0;
+      int32_t emax = 0;
+      for (int32_t s = 0; s < ns; s++) {
+         plan.steps[s].ext0 = (int32_t)total;
+         total += ec[s];
+         plan.steps[s].ext1 = (int32_t)total;
+         emax = std::max(emax, ec[s]);
+      }
+      // a step about 230 ns, a row 0.5, an external entry 3, a part's lag 2200
+      const double ns_est =
+         230.0 * plan.max_steps + (0.5 * (double)n + 3.0 * (double)total) / plan.parts + 2200.0 * plan.parts;
+      if (ns_est >= other_ns || plan.max_steps >= kPipeMaxNeed) return TNLB_OK;
+      const int32_t kk = k <= 4 ? std::max(k, 1) : 8;
+      const int32_t row_bytes = row_size<Upper>(kk);
+      consumers = (plan.max_rows + 31) / 32;
+      // every consumer thread reads its row, also beyond a step's last
+      lay.in_off = kPipeRows0 + consumers * 32 * row_bytes;
+      lay.ext_off = lay.in_off + consumers * 32 * (int32_t)sizeof(Real);
+      const int64_t bytes = (lay.ext_off + (int64_t)emax * (int64_t)sizeof(Real) + 127) / 128 * 128;
+      const int64_t fit = ((int64_t)kPipeSmem - (int64_t)kPipeWindow * (int64_t)sizeof(Real)) / bytes;
+      if (fit < 4) return TNLB_OK;
+      lay.stages = (int32_t)std::min<int64_t>(fit, kPipeMaxStages);
+      lay.stage_bytes = (int32_t)bytes;
+      parts = plan.parts;
+      npad = plan.npad;
+      TNLB_TRY_STATUS(packed.alloc((size_t)npad * row_bytes));
+      TNLB_TRY_STATUS(ext.alloc(sizeof(PipeExt) * (size_t)total));
+      TNLB_CUDA_TRY(cudaMemcpyAsync(steps.ptr, plan.steps.data(), sizeof(PipeStep) * (size_t)ns,
+                                    cudaMemcpyHostToDevice, st));
+      TNLB_CUDA_TRY(cudaMemsetAsync(count.ptr, 0, sizeof(int32_t) * (size_t)ns, st));
+      const unsigned g = grid_for(npad, 256);
+      auto emit = [&](auto* kern) {
+         kern<<<g, 256, 0, st>>>(dev, lay, lu, dst_of, count.as<int32_t>(), packed.as<unsigned char>(), ext.as<PipeExt>());
+      };
+      if (kk == 1) emit(k_pipe_emit<Real, 1, Upper>);
+      else if (kk == 2) emit(k_pipe_emit<Real, 2, Upper>);
+      else if (kk == 3) emit(k_pipe_emit<Real, 3, Upper>);
+      else if (kk == 4) emit(k_pipe_emit<Real, 4, Upper>);
+      else emit(k_pipe_emit<Real, 8, Upper>);
+      TNLB_CHECK_LAUNCH();
+      TNLB_CUDA_TRY(
+         cudaFuncSetAttribute(kernel<Upper>(kk), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPipeSmem));
+      TNLB_CUDA_TRY(cudaStreamSynchronize(st));
+      K = kk;
+      return TNLB_OK;
+   }
+
+   // The plan's steps and row order on the device, as k_pipe_count and
+   // k_pipe_emit read them.
+   tnlb_status upload(const PipePlan& plan, DeviceBuffer& pos, DeviceBuffer& step, cudaStream_t st)
+   {
+      const size_t n = plan.pos.size();
+      auto put = [&](DeviceBuffer& d, const void* h, size_t bytes) -> tnlb_status {
+         TNLB_TRY_STATUS(d.alloc(bytes));
+         TNLB_CUDA_TRY(cudaMemcpyAsync(d.ptr, h, bytes, cudaMemcpyHostToDevice, st));
+         return TNLB_OK;
+      };
+      TNLB_TRY_STATUS(put(steps, plan.steps.data(), sizeof(PipeStep) * plan.steps.size()));
+      TNLB_TRY_STATUS(put(part_step, plan.part_step.data(), sizeof(int32_t) * plan.part_step.size()));
+      TNLB_TRY_STATUS(put(rows_at, plan.rows_at.data(), sizeof(int32_t) * plan.rows_at.size()));
+      TNLB_TRY_STATUS(put(pos, plan.pos.data(), sizeof(int32_t) * n));
+      return put(step, plan.step.data(), sizeof(int32_t) * n);
+   }
+};
+
 struct Ilu0Base {
    virtual ~Ilu0Base() = default;
    virtual tnlb_status apply(const void* b, void* x, cudaStream_t st) = 0;
@@ -303,6 +397,8 @@ struct Ilu0 : Ilu0Base {
    // off-diagonal U entries): strides kl / ku
    int kl = 0, ku = 0;
    DeviceBuffer lpc, lpv, upc, upv, udv, perm;
+   PipeTri<Real> lpipe, upipe;  // the pipelined form of both solves (ilu_pipe.cuh), where it is taken
+   DeviceBuffer lin, uin, progress;
    std::vector<int32_t> lptr, uptr;  // level boundaries into lrows / urows
    cudaGraphExec_t exec = nullptr;
    const Real* g_b = nullptr;
@@ -415,10 +511,23 @@ struct Ilu0 : Ilu0Base {
       }
    }
 
+   // x = U^-1 L^-1 b: b to L's packed order, L's result straight to U's.
+   tnlb_status apply_pipe(const Real* b, Real* x, cudaStream_t st)
+   {
+      int32_t* pr = progress.as<int32_t>();
+      const int32_t flags = (kPipeMaxParts + 1) * 32;
+      k_pipe_start<Real><<<grid_for(std::max(lpipe.npad, 2 * flags), 256), 256, 0, st>>>(
+         lpipe.rows_at.template as<int32_t>(), lpipe.npad, b, lin.as<Real>(), pr, 2 * flags);
+      TNLB_CHECK_LAUNCH();
+      TNLB_TRY_STATUS((lpipe.template launch<false>(lin.as<Real>(), uin.as<Real>(), uin.as<Real>(), pr, st)));
+      return upipe.template launch<true>(uin.as<Real>(), x, x, pr + flags, st);
+   }
+
    tnlb_status apply(const void* bv, void* xv, cudaStream_t st) override
    {
       const Real* b = static_cast<const Real*>(bv);
       Real* x = static_cast<Real*>(xv);
+      if (lpipe.K > 0) return apply_pipe(b, x, st);
       // Solves are replayed from a graph captured for fixed (b, x) buffers:
       // copy in/out of the graph's own buffers when the caller's differ.
       if (!exec) {
@@ -502,6 +611,57 @@ tnlb_status create_from_factors_t(int32_t n, const std::vector<int32_t>& rp, con
    return TNLB_OK;
 }
 
+// The pipelined form of both triangular solves where it is expected to be
+// faster than the level-by-level one, by times measured on 5- and 7-point
+// grids: a level of at most kIluPipeThreads rows 1.0 us, a larger one 2.3 us
+// plus its rows' 60 bytes at 3 TB/s.
+template <typename Real>
+tnlb_status build_pipe(Ilu0<Real>* P, const std::vector<int32_t>& llev, const std::vector<int32_t>& ulev,
+                       int32_t lmax, int32_t umax, int32_t ml, int32_t mu, cudaStream_t st)
+{
+   auto level_ns = [](const std::vector<int32_t>& ptr) {
+      double t = 0;
+      for (size_t l = 0; l + 1 < ptr.size(); l++) {
+         const int32_t rows = ptr[l + 1] - ptr[l];
+         t += rows <= kIluPipeThreads ? 1000.0 : 2300.0 + 0.02 * rows;
+      }
+      return t;
+   };
+   int dev = 0, sms = 0;
+   TNLB_CUDA_TRY(cudaGetDevice(&dev));
+   TNLB_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+   const int32_t parts = pipe_parts(P->n, sms);
+   const double least = 2200.0 * parts + 0.5 * P->n / parts;  // with no level at all
+   if (least >= level_ns(P->lptr) || least >= level_ns(P->uptr)) return TNLB_OK;
+   PipePlan L = pipe_plan(llev, lmax, parts), U = pipe_plan(ulev, umax, parts);
+   DeviceBuffer lpos, lstep, upos, ustep;
+   TNLB_TRY_STATUS(P->lpipe.upload(L, lpos, lstep, st));
+   TNLB_TRY_STATUS(P->upipe.upload(U, upos, ustep, st));
+   const int32_t* cols = P->cols.template as<int32_t>();
+   auto i32 = [](const DeviceBuffer& d) { return d.as<int32_t>(); };
+   const PipeBuild bl{i32(P->lpipe.rows_at), i32(lpos), i32(lstep), i32(P->lstart), i32(P->ustart), cols,
+                      i32(P->lpipe.part_step), P->lpipe.steps.template as<PipeStep>(), L.npad, L.chunk, 0};
+   const PipeBuild bu{i32(P->upipe.rows_at), i32(upos), i32(ustep), i32(P->ustart), i32(P->uend), cols,
+                      i32(P->upipe.part_step), P->upipe.steps.template as<PipeStep>(), U.npad, U.chunk, 1};
+   const Real* lu = P->lu.template as<Real>();
+   TNLB_TRY_STATUS(P->upipe.template build<true>(U, bu, mu, lu, nullptr, level_ns(P->uptr), st));
+   if (P->upipe.K > 0)
+      TNLB_TRY_STATUS(P->lpipe.template build<false>(L, bl, ml, lu, i32(upos), level_ns(P->lptr), st));
+   if (P->lpipe.K == 0) {
+      for (PipeTri<Real>* t : {&P->lpipe, &P->upipe}) {
+         t->K = 0;
+         for (DeviceBuffer* d : {&t->steps, &t->part_step, &t->rows_at, &t->packed, &t->ext}) d->release();
+      }
+      return TNLB_OK;
+   }
+   TNLB_TRY_STATUS(P->lin.alloc(sizeof(Real) * (size_t)L.npad));
+   TNLB_TRY_STATUS(P->uin.alloc(sizeof(Real) * (size_t)U.npad));
+   TNLB_TRY_STATUS(P->progress.alloc(sizeof(int32_t) * 2 * (kPipeMaxParts + 1) * 32));
+   TNLB_CUDA_TRY(cudaMemsetAsync(P->uin.ptr, 0, sizeof(Real) * (size_t)U.npad, st));  // the padding is copied, not used
+   TNLB_CUDA_TRY(cudaStreamSynchronize(st));
+   return TNLB_OK;
+}
+
 // L/U split, dependency levels, level order and packed copies of the factors;
 // with `factorize`, the ILU(0) factorisation of P->lu in place first.
 template <typename Real>
@@ -511,6 +671,7 @@ tnlb_status analyze_t(Ilu0<Real>* P, const std::vector<int32_t>& rp, const std::
    const int32_t n = P->n;
    std::vector<int32_t> ls(n), us(n), ue(n), llev(n, 0), ulev(n, 0);
    int32_t lmax = 0, umax = 0;
+   bool ordered = true;  // every off-diagonal entry of U lies right of its row
    for (int32_t i = 0; i < n; i++) {
       int32_t c = rp[i];
       // ILU0.hpp:35-55: columns < i -> L, i <= column < N -> U (sorted rows)
@@ -526,7 +687,10 @@ tnlb_status analyze_t(Ilu0<Real>* P, const std::vector<int32_t>& rp, const std::
    }
    for (int32_t i = n - 1; i >= 0; i--) {
       int32_t lv = 0;
-      for (int32_t q = us[i] + 1; q < ue[i]; q++) lv = std::max(lv, ulev[cols[q]] + 1);
+      for (int32_t q = us[i] + 1; q < ue[i]; q++) {
+         lv = std::max(lv, ulev[cols[q]] + 1);
+         ordered = ordered && cols[q] > i;
+      }
       ulev[i] = lv;
       umax = std::max(umax, lv);
    }
@@ -571,6 +735,11 @@ tnlb_status analyze_t(Ilu0<Real>* P, const std::vector<int32_t>& rp, const std::
    for (int32_t i = 0; i < n; i++) {
       ml = std::max(ml, us[i] - ls[i]);
       mu = std::max(mu, ue[i] - us[i] - 1);
+   }
+   if (ml <= 8 && mu <= 8 && ordered) TNLB_TRY_STATUS(build_pipe(P, llev, ulev, lmax, umax, ml, mu, st));
+   if (P->lpipe.K > 0) {
+      for (DeviceBuffer* d : {&P->lrows, &P->urows, &P->dlptr, &P->duptr}) d->release();
+      return TNLB_OK;
    }
    if (ml <= 8 && mu <= 8) {
       auto stride = [](int32_t m) { return m <= 1 ? 1 : m <= 2 ? 2 : m <= 4 ? 4 : 8; };
