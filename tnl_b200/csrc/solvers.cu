@@ -24,31 +24,9 @@
 #include "segview.cuh"
 #include "compact.cuh"
 #include "band.cuh"
+#include "persist.cuh"
 
 namespace tnlb {
-
-// Device-resident solver scalars.
-struct DevState {
-   double normb, s1, s2, alpha, beta, omega, rho, rho_old, r_ast_sqnorm, residue;
-   double conv, div;
-   int32_t it, done, maxit, minit;
-   int32_t flag;
-   uint32_t loops;  // bodies run by the current launch of a looping iteration graph
-};
-
-__device__ __forceinline__ bool check_next(const DevState& S)
-{
-   return !(isnan(S.residue) || S.it > S.maxit || (S.residue > S.div && S.it >= S.minit) ||
-            (S.residue < S.conv && S.it >= S.minit));
-}
-
-// IterativeSolver::nextIteration (IterativeSolver.hpp:98-108).
-__device__ __forceinline__ void next_iteration(DevState& S)
-{
-   const bool c = check_next(S);
-   S.it++;
-   if (!c) S.done = 1;
-}
 
 // IterativeSolver::checkConvergence (IterativeSolver.hpp:121-143).
 static bool check_convergence(double residue, int it, int maxit, int minit, double conv, double div)
@@ -658,6 +636,32 @@ struct Ctx {
    }
 };
 
+// Iterations per launch of a resident solver kernel: it ends from time to time
+// however many iterations the caller allows.
+constexpr int32_t kPersistCap = 2048;
+
+// Runs a resident solver kernel (persist.cuh) until the state is done and reads
+// it back.  `args`: the kernel's arguments up to n.
+tnlb_status persist_run(const void* kern, const PersistShape& sh, std::vector<void*> args, int32_t n, const Work& W,
+                        cudaStream_t st, DevState* h)
+{
+   DeviceBuffer sync;
+   TNLB_TRY_STATUS(sync.alloc(kPersistSlotBytes + sizeof(int32_t)));
+   PersistSync g = persist_sync(sync);
+   DevState* S = W.S();
+   int32_t cap = kPersistCap, err = 0;
+   for (void* a : {(void*)&n, (void*)&S, (void*)&g, (void*)&cap}) args.push_back(a);
+   do {
+      TNLB_CUDA_TRY(cudaMemsetAsync(sync.ptr, 0, sync.bytes, st));
+      TNLB_CUDA_TRY(cudaLaunchCooperativeKernel(kern, dim3(sh.blocks), dim3(sh.threads), args.data(), sh.smem, st));
+      TNLB_CUDA_TRY(cudaMemcpyAsync(h, S, sizeof(*h), cudaMemcpyDeviceToHost, st));
+      TNLB_CUDA_TRY(cudaMemcpyAsync(&err, g.err, sizeof(err), cudaMemcpyDeviceToHost, st));
+      TNLB_CUDA_TRY(cudaStreamSynchronize(st));
+      TNLB_REQUIRE(err == 0, TNLB_ERR_CUDA, "solver kernel: a wait between blocks ran out");
+   } while (!h->done);
+   return TNLB_OK;
+}
+
 // ------------------------------------------------------------------ CG
 
 template <typename Real>
@@ -705,6 +709,19 @@ tnlb_status cg_solve(const Ctx<Real>& c, const Precond<Real>& P, const tnlb_solv
    else
       k_cg_init<Real><<<G, kRedThreads, 0, c.st>>>(n, r.as<Real>(), z.as<Real>(), p.as<Real>(), P.d(), W.red(), W.S());
    TNLB_CHECK_LAUNCH();
+   const void* kern = persist_rows_fit(c.seg) && !gen ? persist_pick<Real, CgPersistKernel>(c.seg) : nullptr;
+   PersistShape sh;
+   if (kern && persist_shape(kern, (int32_t)n, 4, sizeof(Real), sh)) {
+      PersistVectors<Real, 4> V{{Ap.as<Real>(), r.as<Real>(), x, const_cast<Real*>(P.d())}, sh.kept, sh.rows};
+      PersistRows<Real> A = persist_rows(c.seg, c.cols, c.vals);
+      Real* pp = p.as<Real>();
+      TNLB_TRY_STATUS(persist_run(kern, sh, {&A, &V, &pp}, (int32_t)n, W, c.st, &h));
+      res->iterations = h.it;
+      res->residue = h.residue;
+      res->converged = check_convergence(h.residue, h.it, h.maxit, h.minit, h.conv, h.div);
+      res->status_detail = 0;
+      return TNLB_OK;
+   }
    // One iteration (CG.hpp:60-107): every kernel returns at once when the
    // device `done` flag is set, so batches may run past the stopping point.
    // short-row CSR: (p, Ap) summed inside the product's kernel
@@ -861,6 +878,7 @@ tnlb_status pcg_general(const Ctx<Real>& c, const Precond<Real>& P, const tnlb_s
    normb = std::sqrt(normb);
    if (normb == 0) {
       TNLB_CUDA_TRY(cudaMemsetAsync(x, 0, sizeof(Real) * n, c.st));
+      TNLB_CUDA_TRY(cudaStreamSynchronize(c.st));
       *res = tnlb_solve_result{1, 0, 0.0, 0, 0};
       return TNLB_OK;
    }
@@ -952,6 +970,7 @@ tnlb_status bicgstab_solve(const Ctx<Real>& c, const Precond<Real>& P, const tnl
    b_norm = std::sqrt(hs[0]);
    if (b_norm == 0) {
       TNLB_CUDA_TRY(cudaMemsetAsync(x, 0, sizeof(Real) * n, c.st));
+      TNLB_CUDA_TRY(cudaStreamSynchronize(c.st));
       *res = tnlb_solve_result{1, 0, 0.0, 0, 0};
       return TNLB_OK;
    }
@@ -964,7 +983,52 @@ tnlb_status bicgstab_solve(const Ctx<Real>& c, const Precond<Real>& P, const tnl
    const double eps2 = DBL_EPSILON * DBL_EPSILON;
    const double eps2r = (sizeof(Real) == 4) ? (double)FLT_EPSILON * FLT_EPSILON : eps2;
    residue = std::sqrt(rho) / b_norm;
-   while (true) {
+   // rho too small against |r_ast|^2: r, r_ast and rho afresh (BICGStab.hpp:96-104)
+   double rnorm2 = 0;
+   auto restart = [&]() -> tnlb_status {
+      TNLB_TRY_STATUS(compute_residue(r.as<Real>()));
+      TNLB_CUDA_TRY(cudaMemcpyAsync(r_ast.ptr, r.ptr, sizeof(Real) * n, cudaMemcpyDeviceToDevice, c.st));
+      TNLB_TRY_STATUS(dots(r.as<Real>(), r_ast.as<Real>(), nullptr, nullptr));
+      r_ast_sqnorm = rho = hs[0];
+      rnorm2 = hs[0];
+      return TNLB_OK;
+   };
+   const bool diagonal = P.kind == TNLB_PRECOND_NONE || P.kind == TNLB_PRECOND_JACOBI;
+   const void* kern = diagonal && !prm.bicgstab_exact_residue && persist_rows_fit(c.seg)
+                         ? persist_pick<Real, BicgPersistKernel>(c.seg)
+                         : nullptr;
+   PersistShape sh;
+   const bool persist = kern && persist_shape(kern, (int32_t)n, 6, sizeof(Real), sh);
+   if (persist) {
+      PersistVectors<Real, 6> V{{Ap.as<Real>(), r.as<Real>(), As.as<Real>(), r_ast.as<Real>(), x,
+                                 const_cast<Real*>(P.d())},
+                                sh.kept,
+                                sh.rows};
+      PersistRows<Real> A = persist_rows(c.seg, c.cols, c.vals);
+      Real *pp = p.as<Real>(), *ps = s.as<Real>();
+      DevState h = initial_state(prm);
+      h.normb = b_norm;
+      h.rho = rho;
+      h.r_ast_sqnorm = r_ast_sqnorm;
+      h.residue = residue;
+      while (h.done != 1) {
+         h.done = 0;
+         TNLB_CUDA_TRY(cudaMemcpyAsync(W.S(), &h, sizeof(h), cudaMemcpyHostToDevice, c.st));
+         TNLB_TRY_STATUS(persist_run(kern, sh, {&A, &V, &pp, &ps}, (int32_t)n, W, c.st, &h));
+         if (h.done != kPersistRestart) continue;
+         TNLB_TRY_STATUS(restart());
+         h.beta = (rho / h.rho_old) * (h.alpha / h.omega);
+         k_bicg_p<Real><<<G, kRedThreads, 0, c.st>>>(n, p.as<Real>(), r.as<Real>(), Ap.as<Real>(), (Real)h.beta,
+                                                     (Real)(h.beta * h.omega));
+         TNLB_CHECK_LAUNCH();
+         h.rho = rho;
+         h.r_ast_sqnorm = r_ast_sqnorm;
+         h.residue = std::sqrt(rnorm2) / b_norm;
+      }
+      it = h.it;
+      residue = h.residue;
+   }
+   while (!persist) {
       const bool cont = check();
       it++;
       if (!cont) break;
@@ -985,15 +1049,9 @@ tnlb_status bicgstab_solve(const Ctx<Real>& c, const Precond<Real>& P, const tnl
       TNLB_CUDA_TRY(cudaStreamSynchronize(c.st));
       const double rho_old = rho;
       rho = hs[0];
-      double rnorm2 = hs[1];
+      rnorm2 = hs[1];
       (void)eps2r;
-      if (std::fabs(rho) < eps2 * r_ast_sqnorm) {
-         TNLB_TRY_STATUS(compute_residue(r.as<Real>()));
-         TNLB_CUDA_TRY(cudaMemcpyAsync(r_ast.ptr, r.ptr, sizeof(Real) * n, cudaMemcpyDeviceToDevice, c.st));
-         TNLB_TRY_STATUS(dots(r.as<Real>(), r_ast.as<Real>(), nullptr, nullptr));
-         r_ast_sqnorm = rho = hs[0];
-         rnorm2 = hs[0];
-      }
+      if (std::fabs(rho) < eps2 * r_ast_sqnorm) TNLB_TRY_STATUS(restart());
       const double beta = (rho / rho_old) * (alpha / omega);
       k_bicg_p<Real><<<G, kRedThreads, 0, c.st>>>(n, p.as<Real>(), r.as<Real>(), Ap.as<Real>(), (Real)beta,
                                                   (Real)(beta * omega));
@@ -1339,6 +1397,7 @@ tnlb_status gmres_solve(const Ctx<Real>& c, const Precond<Real>& P, const tnlb_s
       TNLB_TRY_STATUS(norm(b, &normb));
    if (normb == 0) {
       TNLB_CUDA_TRY(cudaMemsetAsync(x, 0, sizeof(Real) * n, c.st));
+      TNLB_CUDA_TRY(cudaStreamSynchronize(c.st));
       *res = tnlb_solve_result{1, 0, 0.0, 0, 0};
       return TNLB_OK;
    }
