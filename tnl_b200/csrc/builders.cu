@@ -379,11 +379,11 @@ tnlb_status build_acsr(tnlb_segments* seg, cudaStream_t stream)
    for (int k = 0; k < 6; k++) seg->acsr_count[k] = 0;
    if (n == 0 || seg->max_size == 0) return TNLB_OK;  // max(offsets) == 0: blocks reset
    DeviceBuffer end, type, starts, base, counts;
-   TNLB_TRY_STATUS(end.alloc(sizeof(int32_t) * n));
-   TNLB_TRY_STATUS(type.alloc(n));
-   TNLB_TRY_STATUS(starts.alloc(sizeof(int32_t) * n));
-   TNLB_TRY_STATUS(base.alloc(sizeof(int64_t) * n));
-   TNLB_TRY_STATUS(counts.alloc(sizeof(int64_t) * 2));
+   TNLB_TRY_STATUS(end.alloc(sizeof(int32_t) * n, stream));
+   TNLB_TRY_STATUS(type.alloc(n, stream));
+   TNLB_TRY_STATUS(starts.alloc(sizeof(int32_t) * n, stream));
+   TNLB_TRY_STATUS(base.alloc(sizeof(int64_t) * n, stream));
+   TNLB_TRY_STATUS(counts.alloc(sizeof(int64_t) * 2, stream));
    for (int k = 0; k < 6; k++) {
       const int64_t sizeOfValue = 1 << k;
       const int64_t limit = (24576 / sizeOfValue) / 8;
@@ -425,11 +425,11 @@ tnlb_status build_chell(tnlb_segments* seg, const int32_t* d_sizes, cudaStream_t
       return TNLB_OK;
    }
    DeviceBuffer P, end, starts, counts, storage_raw;
-   TNLB_TRY_STATUS(P.alloc(sizeof(int32_t) * ((size_t)n + 1)));
+   TNLB_TRY_STATUS(P.alloc(sizeof(int32_t) * ((size_t)n + 1), stream));
    TNLB_TRY_STATUS(exclusive_scan_i32(d_sizes, P.as<int32_t>(), n, nullptr, stream, true));
-   TNLB_TRY_STATUS(end.alloc(sizeof(int32_t) * n));
-   TNLB_TRY_STATUS(starts.alloc(sizeof(int32_t) * n));
-   TNLB_TRY_STATUS(counts.alloc(sizeof(int64_t) * 2));
+   TNLB_TRY_STATUS(end.alloc(sizeof(int32_t) * n, stream));
+   TNLB_TRY_STATUS(starts.alloc(sizeof(int32_t) * n, stream));
+   TNLB_TRY_STATUS(counts.alloc(sizeof(int64_t) * 2, stream));
    k_chell_end<<<grid_for(n, 256), 256, 0, stream>>>(P.as<int32_t>(), n, end.as<int32_t>());
    TNLB_CHECK_LAUNCH();
    k_chain_walk<<<1, 1024, 0, stream>>>(end.as<int32_t>(), nullptr, n, starts.as<int32_t>(), nullptr,
@@ -444,7 +444,7 @@ tnlb_status build_chell(tnlb_segments* seg, const int32_t* d_sizes, cudaStream_t
    TNLB_TRY_STATUS(seg->ch_slice_chunk_size.alloc(sizeof(int32_t) * slices));
    TNLB_TRY_STATUS(seg->ch_slice_first.alloc(sizeof(int32_t) * slices));
    TNLB_TRY_STATUS(seg->ch_slice_pointer.alloc(sizeof(int32_t) * ((size_t)slices + 1)));
-   TNLB_TRY_STATUS(storage_raw.alloc(sizeof(int32_t) * slices));
+   TNLB_TRY_STATUS(storage_raw.alloc(sizeof(int32_t) * slices, stream));
    k_chell_slice<<<slices, kChunksInSlice, 0, stream>>>(
       d_sizes, P.as<int32_t>(), starts.as<int32_t>(), slices, n, seg->ch_slice_size.as<int32_t>(),
       seg->ch_slice_first.as<int32_t>(), seg->ch_slice_chunk_size.as<int32_t>(), storage_raw.as<int32_t>(),
@@ -516,7 +516,7 @@ tnlb_status build_segments(tnlb_segments* seg, const int32_t* d_sizes, cudaStrea
          TNLB_TRY_STATUS(seg->slice_offsets.alloc(sizeof(int32_t) * ((size_t)slices + 1)));
          TNLB_TRY_STATUS(seg->slice_segment_sizes.alloc(sizeof(int32_t) * (size_t)slices));
          DeviceBuffer raw;
-         TNLB_TRY_STATUS(raw.alloc(sizeof(int32_t) * (size_t)slices));
+         TNLB_TRY_STATUS(raw.alloc(sizeof(int32_t) * (size_t)slices, stream));
          if (slices > 0) {
             k_sell_slice_max<<<grid_for((int64_t)slices * 32, 256), 256, 0, stream>>>(
                d_sizes, n, slices, seg->slice_segment_sizes.as<int32_t>(), raw.as<int32_t>());
@@ -534,7 +534,7 @@ tnlb_status build_segments(tnlb_segments* seg, const int32_t* d_sizes, cudaStrea
          TNLB_TRY_STATUS(seg->bi_perm.alloc(sizeof(int32_t) * (size_t)n));
          TNLB_TRY_STATUS(seg->bi_group_pointers.alloc(sizeof(int32_t) * ((size_t)strips * kBiGroups + 1)));
          DeviceBuffer raw;
-         TNLB_TRY_STATUS(raw.alloc(sizeof(int32_t) * ((size_t)strips * kBiGroups)));
+         TNLB_TRY_STATUS(raw.alloc(sizeof(int32_t) * ((size_t)strips * kBiGroups), stream));
          if (strips > 0) {
             k_biell_strips<<<grid_for(strips, 8), 256, 0, stream>>>(d_sizes, n, strips, seg->bi_perm.as<int32_t>(),
                                                                      raw.as<int32_t>());

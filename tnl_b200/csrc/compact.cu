@@ -172,7 +172,7 @@ tnlb_status row_excess(const int32_t* rowptr, const int32_t* cols, const double*
                        DeviceBuffer* s, bool* ok)
 {
    DeviceBuffer bad;
-   TNLB_TRY_STATUS(bad.alloc(sizeof(int32_t)));
+   TNLB_TRY_STATUS(bad.alloc(sizeof(int32_t), st));
    TNLB_TRY_STATUS(s->alloc(sizeof(float) * (n > 0 ? n : 1)));
    TNLB_CUDA_TRY(cudaMemsetAsync(bad.ptr, 0, sizeof(int32_t), st));
    k_row_excess<<<grid_for(n, 256), 256, 0, st>>>(rowptr, cols, v, n, s->as<float>(), bad.as<int32_t>());
@@ -285,7 +285,7 @@ tnlb_status diag_build(const tnlb_segments* seg, const int32_t* cols, const floa
    if (n <= 0 || nnz <= 0) return TNLB_OK;
    const int32_t* rp = seg->offsets.as<int32_t>();
    DeviceBuffer tab;
-   TNLB_TRY_STATUS(tab.alloc(sizeof(int32_t) * (kDiagSlots + 1)));
+   TNLB_TRY_STATUS(tab.alloc(sizeof(int32_t) * (kDiagSlots + 1), st));
    int32_t* flag = tab.as<int32_t>() + kDiagSlots;
    k_diag_table_init<<<1, 32, 0, st>>>(tab.as<int32_t>(), flag);
    TNLB_CHECK_LAUNCH();
@@ -345,7 +345,7 @@ tnlb_status half_scale(const float* vals, int64_t nnz, cudaStream_t st, float* s
    *scale = 1.0f;
    if (nnz <= 0) return TNLB_OK;
    DeviceBuffer m;
-   TNLB_TRY_STATUS(m.alloc(sizeof(unsigned)));
+   TNLB_TRY_STATUS(m.alloc(sizeof(unsigned), st));
    TNLB_CUDA_TRY(cudaMemsetAsync(m.ptr, 0, sizeof(unsigned), st));
    k_absmax<<<grid_for(nnz, 256 * 8), 256, 0, st>>>(vals, nnz, m.as<unsigned>());
    TNLB_CHECK_LAUNCH();
@@ -391,7 +391,7 @@ tnlb_status compact_build(const tnlb_segments* seg, const int32_t* cols, const f
    out->rowptr = seg->offsets.as<int32_t>();
    out->half = half;
    DeviceBuffer bad;
-   TNLB_TRY_STATUS(bad.alloc(sizeof(int32_t)));
+   TNLB_TRY_STATUS(bad.alloc(sizeof(int32_t), st));
    TNLB_CUDA_TRY(cudaMemsetAsync(bad.ptr, 0, sizeof(int32_t), st));
    TNLB_TRY_STATUS(out->off.alloc(sizeof(int16_t) * (nnz > 0 ? nnz : 1)));
    k_rel_offsets<<<grid_for(n, 256), 256, 0, st>>>(out->rowptr, cols, n, out->off.as<int16_t>(), bad.as<int32_t>());

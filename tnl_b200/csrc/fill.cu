@@ -142,7 +142,7 @@ tnlb_status fill_from_csr(const tnlb_segments* seg, tnlb_real real, const int32_
    }
    if (seg->n == 0) return TNLB_OK;
    DeviceBuffer err;
-   TNLB_TRY_STATUS(err.alloc(sizeof(int32_t)));
+   TNLB_TRY_STATUS(err.alloc(sizeof(int32_t), stream));
    TNLB_CUDA_TRY(cudaMemsetAsync(err.ptr, 0, sizeof(int32_t), stream));
    const SegView v = view_of(seg);
    if (real == TNLB_F64)

@@ -143,7 +143,7 @@ tnlb_status scan_totals(int64_t* d, int64_t n, cudaStream_t stream)
       return TNLB_OK;
    }
    DeviceBuffer t;
-   TNLB_TRY_STATUS(t.alloc(sizeof(int64_t) * blocks));
+   TNLB_TRY_STATUS(t.alloc(sizeof(int64_t) * blocks, stream));
    k_block_totals<int64_t><<<(unsigned)blocks, kScanThreads, 0, stream>>>(d, n, t.as<int64_t>());
    TNLB_CHECK_LAUNCH();
    TNLB_TRY_STATUS(scan_totals(t.as<int64_t>(), blocks, stream));
@@ -160,10 +160,10 @@ tnlb_status scan_i32(const int32_t* d_in, int32_t* d_out, int64_t n, int64_t* h_
 {
    const int64_t blocks = (n + kScanTile - 1) / kScanTile;
    DeviceBuffer totals, grand;
-   TNLB_TRY_STATUS(grand.alloc(sizeof(int64_t)));
+   TNLB_TRY_STATUS(grand.alloc(sizeof(int64_t), stream));
    TNLB_CUDA_TRY(cudaMemsetAsync(grand.ptr, 0, sizeof(int64_t), stream));
    if (n > 0) {
-      TNLB_TRY_STATUS(totals.alloc(sizeof(int64_t) * blocks));
+      TNLB_TRY_STATUS(totals.alloc(sizeof(int64_t) * blocks, stream));
       k_block_totals<int32_t><<<(unsigned)blocks, kScanThreads, 0, stream>>>(d_in, n, totals.as<int64_t>());
       TNLB_CHECK_LAUNCH();
       TNLB_TRY_STATUS(scan_totals(totals.as<int64_t>(), blocks, stream));
@@ -201,7 +201,7 @@ tnlb_status inclusive_scan_i32_inplace(int32_t* d_data, int64_t n, cudaStream_t 
 tnlb_status reduce_max_i32(const int32_t* d_in, int64_t n, int32_t* h_max, cudaStream_t stream)
 {
    DeviceBuffer m;
-   TNLB_TRY_STATUS(m.alloc(sizeof(int32_t)));
+   TNLB_TRY_STATUS(m.alloc(sizeof(int32_t), stream));
    TNLB_CUDA_TRY(cudaMemsetAsync(m.ptr, 0, sizeof(int32_t), stream));
    if (n > 0) {
       unsigned g = grid_for(n, kScanThreads * 8);
@@ -217,7 +217,7 @@ tnlb_status reduce_max_i32(const int32_t* d_in, int64_t n, int32_t* h_max, cudaS
 tnlb_status reduce_sum_i64(const int32_t* d_in, int64_t n, int64_t* h_sum, cudaStream_t stream)
 {
    DeviceBuffer tmp;
-   TNLB_TRY_STATUS(tmp.alloc(sizeof(int32_t) * (n + 1)));
+   TNLB_TRY_STATUS(tmp.alloc(sizeof(int32_t) * (n + 1), stream));
    return exclusive_scan_i32(d_in, tmp.as<int32_t>(), n, h_sum, stream, false);
 }
 

@@ -527,13 +527,13 @@ Precond<Real> view(const tnlb_precond* P)
 
 struct Work {
    DeviceBuffer state, partials, counter, scratch;
-   tnlb_status alloc()
+   tnlb_status alloc(cudaStream_t st)
    {
-      TNLB_TRY_STATUS(state.alloc(sizeof(DevState)));
-      TNLB_TRY_STATUS(partials.alloc(sizeof(double) * kRedMaxBlocks * 64));
-      TNLB_TRY_STATUS(counter.alloc(sizeof(unsigned) * 4));
-      TNLB_TRY_STATUS(scratch.alloc(sizeof(double) * 256));
-      TNLB_CUDA_TRY(cudaMemset(counter.ptr, 0, sizeof(unsigned) * 4));
+      TNLB_TRY_STATUS(state.alloc(sizeof(DevState), st));
+      TNLB_TRY_STATUS(partials.alloc(sizeof(double) * kRedMaxBlocks * 64, st));
+      TNLB_TRY_STATUS(counter.alloc(sizeof(unsigned) * 4, st));
+      TNLB_TRY_STATUS(scratch.alloc(sizeof(double) * 256, st));
+      TNLB_CUDA_TRY(cudaMemsetAsync(counter.ptr, 0, sizeof(unsigned) * 4, st));
       return TNLB_OK;
    }
    RedWork red() const { return {partials.as<double>(), counter.as<unsigned>()}; }
@@ -646,7 +646,7 @@ tnlb_status persist_run(const void* kern, const PersistShape& sh, std::vector<vo
                         cudaStream_t st, DevState* h)
 {
    DeviceBuffer sync;
-   TNLB_TRY_STATUS(sync.alloc(kPersistSlotBytes + sizeof(int32_t)));
+   TNLB_TRY_STATUS(sync.alloc(kPersistSlotBytes + sizeof(int32_t), st));
    PersistSync g = persist_sync(sync);
    DevState* S = W.S();
    int32_t cap = kPersistCap, err = 0;
@@ -670,12 +670,12 @@ tnlb_status cg_solve(const Ctx<Real>& c, const Precond<Real>& P, const tnlb_solv
 {
    const int64_t n = c.n;
    Work W;
-   TNLB_TRY_STATUS(W.alloc());
+   TNLB_TRY_STATUS(W.alloc(c.st));
    DeviceBuffer r, p, Ap, z;
-   TNLB_TRY_STATUS(r.alloc(sizeof(Real) * n));
-   TNLB_TRY_STATUS(p.alloc(sizeof(Real) * n));
-   TNLB_TRY_STATUS(Ap.alloc(sizeof(Real) * n));
-   TNLB_TRY_STATUS(z.alloc(sizeof(Real) * n));
+   TNLB_TRY_STATUS(r.alloc(sizeof(Real) * n, c.st));
+   TNLB_TRY_STATUS(p.alloc(sizeof(Real) * n, c.st));
+   TNLB_TRY_STATUS(Ap.alloc(sizeof(Real) * n, c.st));
+   TNLB_TRY_STATUS(z.alloc(sizeof(Real) * n, c.st));
    DevState s0 = initial_state(prm);
    TNLB_CUDA_TRY(cudaMemcpyAsync(W.S(), &s0, sizeof(s0), cudaMemcpyHostToDevice, c.st));
    const unsigned G = vec_grid(n);
@@ -728,9 +728,9 @@ tnlb_status cg_solve(const Ctx<Real>& c, const Precond<Real>& P, const tnlb_solv
    const bool fused = spmv_dot_fusable(c.seg);
    DeviceBuffer dot_parts, dot_ctr, dot_val;
    if (fused) {
-      TNLB_TRY_STATUS(dot_parts.alloc(sizeof(double) * spmv_dot_partials(c.seg)));
-      TNLB_TRY_STATUS(dot_ctr.alloc(sizeof(unsigned)));
-      TNLB_TRY_STATUS(dot_val.alloc(sizeof(double)));
+      TNLB_TRY_STATUS(dot_parts.alloc(sizeof(double) * spmv_dot_partials(c.seg), c.st));
+      TNLB_TRY_STATUS(dot_ctr.alloc(sizeof(unsigned), c.st));
+      TNLB_TRY_STATUS(dot_val.alloc(sizeof(double), c.st));
       TNLB_CUDA_TRY(cudaMemsetAsync(dot_ctr.ptr, 0, sizeof(unsigned), c.st));
    }
    const unsigned Gs2 = resident_grid((const void*)k_cg_s2<Real>, kRedThreads, n, 4);
@@ -843,12 +843,12 @@ tnlb_status pcg_general(const Ctx<Real>& c, const Precond<Real>& P, const tnlb_s
 {
    const int64_t n = c.n;
    Work W;
-   TNLB_TRY_STATUS(W.alloc());
+   TNLB_TRY_STATUS(W.alloc(c.st));
    DeviceBuffer r, p, Ap, z;
-   TNLB_TRY_STATUS(r.alloc(sizeof(Real) * n));
-   TNLB_TRY_STATUS(p.alloc(sizeof(Real) * n));
-   TNLB_TRY_STATUS(Ap.alloc(sizeof(Real) * n));
-   TNLB_TRY_STATUS(z.alloc(sizeof(Real) * n));
+   TNLB_TRY_STATUS(r.alloc(sizeof(Real) * n, c.st));
+   TNLB_TRY_STATUS(p.alloc(sizeof(Real) * n, c.st));
+   TNLB_TRY_STATUS(Ap.alloc(sizeof(Real) * n, c.st));
+   TNLB_TRY_STATUS(z.alloc(sizeof(Real) * n, c.st));
    double* sc = W.scratch.as<double>();
    const unsigned G = vec_grid(n);
    double hs[2];
@@ -925,9 +925,9 @@ tnlb_status bicgstab_solve(const Ctx<Real>& c, const Precond<Real>& P, const tnl
 {
    const int64_t n = c.n;
    Work W;
-   TNLB_TRY_STATUS(W.alloc());
+   TNLB_TRY_STATUS(W.alloc(c.st));
    DeviceBuffer r, r_ast, p, s, Ap, As, M_tmp;
-   for (auto* v : {&r, &r_ast, &p, &s, &Ap, &As, &M_tmp}) TNLB_TRY_STATUS(v->alloc(sizeof(Real) * n));
+   for (auto* v : {&r, &r_ast, &p, &s, &Ap, &As, &M_tmp}) TNLB_TRY_STATUS(v->alloc(sizeof(Real) * n, c.st));
    double* sc = W.scratch.as<double>();
    const unsigned G = vec_grid(n);
    double hs[2];
@@ -1126,17 +1126,17 @@ tnlb_status gmres_cwy_solve(const Ctx<Real>& c, const Precond<Real>& P, const tn
                 "GMRES CWY needs at least restarting_max + 1 rows (the reference copies that many entries of Y)");
    const int64_t ld = (n + 31) / 32 * 32;
    Work W;
-   TNLB_TRY_STATUS(W.alloc());
+   TNLB_TRY_STATUS(W.alloc(c.st));
    DeviceBuffer Yb, z, w, v, r, M_tmp, hdev, cdev, ydev;
-   TNLB_TRY_STATUS(Yb.alloc(sizeof(Real) * ld * L));
-   TNLB_TRY_STATUS(z.alloc(sizeof(Real) * n));
-   TNLB_TRY_STATUS(w.alloc(sizeof(Real) * n));
-   TNLB_TRY_STATUS(v.alloc(sizeof(Real) * n));
-   TNLB_TRY_STATUS(r.alloc(sizeof(Real) * n));
-   TNLB_TRY_STATUS(M_tmp.alloc(sizeof(Real) * n));
-   TNLB_TRY_STATUS(hdev.alloc(sizeof(double) * 128));
-   TNLB_TRY_STATUS(cdev.alloc(sizeof(double) * 128));
-   TNLB_TRY_STATUS(ydev.alloc(sizeof(double) * 128));
+   TNLB_TRY_STATUS(Yb.alloc(sizeof(Real) * ld * L, c.st));
+   TNLB_TRY_STATUS(z.alloc(sizeof(Real) * n, c.st));
+   TNLB_TRY_STATUS(w.alloc(sizeof(Real) * n, c.st));
+   TNLB_TRY_STATUS(v.alloc(sizeof(Real) * n, c.st));
+   TNLB_TRY_STATUS(r.alloc(sizeof(Real) * n, c.st));
+   TNLB_TRY_STATUS(M_tmp.alloc(sizeof(Real) * n, c.st));
+   TNLB_TRY_STATUS(hdev.alloc(sizeof(double) * 128, c.st));
+   TNLB_TRY_STATUS(cdev.alloc(sizeof(double) * 128, c.st));
+   TNLB_TRY_STATUS(ydev.alloc(sizeof(double) * 128, c.st));
    Real* Y = Yb.as<Real>();
    double* sc = W.scratch.as<double>();
    const unsigned G = vec_grid(n);
@@ -1350,16 +1350,16 @@ tnlb_status gmres_solve(const Ctx<Real>& c, const Precond<Real>& P, const tnlb_s
    const int m_max = rmax;
    const int64_t ld = (n + 31) / 32 * 32;  // 256-byte aligned columns in FP64
    Work W;
-   TNLB_TRY_STATUS(W.alloc());
+   TNLB_TRY_STATUS(W.alloc(c.st));
    DeviceBuffer V, w, r, M_tmp, hdev, ydev;
-   TNLB_TRY_STATUS(V.alloc(sizeof(Real) * ld * (m_max + 1)));
-   TNLB_TRY_STATUS(w.alloc(sizeof(Real) * n));
-   TNLB_TRY_STATUS(r.alloc(sizeof(Real) * n));
-   TNLB_TRY_STATUS(M_tmp.alloc(sizeof(Real) * n));
-   TNLB_TRY_STATUS(hdev.alloc(sizeof(double) * 128));
-   TNLB_TRY_STATUS(ydev.alloc(sizeof(double) * 128));
+   TNLB_TRY_STATUS(V.alloc(sizeof(Real) * ld * (m_max + 1), c.st));
+   TNLB_TRY_STATUS(w.alloc(sizeof(Real) * n, c.st));
+   TNLB_TRY_STATUS(r.alloc(sizeof(Real) * n, c.st));
+   TNLB_TRY_STATUS(M_tmp.alloc(sizeof(Real) * n, c.st));
+   TNLB_TRY_STATUS(hdev.alloc(sizeof(double) * 128, c.st));
+   TNLB_TRY_STATUS(ydev.alloc(sizeof(double) * 128, c.st));
    DeviceBuffer Z;
-   if (flexible) TNLB_TRY_STATUS(Z.alloc(sizeof(Real) * ld * m_max));
+   if (flexible) TNLB_TRY_STATUS(Z.alloc(sizeof(Real) * ld * m_max, c.st));
    Real* Vp = V.as<Real>();
    double* sc = W.scratch.as<double>();
    const unsigned G = vec_grid(n);
@@ -1653,9 +1653,9 @@ tnlb_status tfqmr_solve(const Ctx<Real>& c, const Precond<Real>& P, const tnlb_s
 {
    const int64_t n = c.n;
    Work W;
-   TNLB_TRY_STATUS(W.alloc());
+   TNLB_TRY_STATUS(W.alloc(c.st));
    DeviceBuffer d, r, w, u, v, r_ast, Au, M_tmp;
-   for (auto* q : {&d, &r, &w, &u, &v, &r_ast, &Au, &M_tmp}) TNLB_TRY_STATUS(q->alloc(sizeof(Real) * n));
+   for (auto* q : {&d, &r, &w, &u, &v, &r_ast, &Au, &M_tmp}) TNLB_TRY_STATUS(q->alloc(sizeof(Real) * n, c.st));
    VecOps<Real> V(c, W);
    const bool pre = P.kind != TNLB_PRECOND_NONE;
    auto pmv = [&](const Real* src, Real* dst) -> tnlb_status {
@@ -1743,12 +1743,12 @@ tnlb_status bicgstabl_solve(const Ctx<Real>& c, const Precond<Real>& P, const tn
    TNLB_REQUIRE(ell >= 1 && ell <= 32, TNLB_ERR_INVALID_ARGUMENT, "bicgstab-ell must lie in 1..32");
    const int64_t ld = (n + 31) / 32 * 32;
    Work W;
-   TNLB_TRY_STATUS(W.alloc());
+   TNLB_TRY_STATUS(W.alloc(c.st));
    DeviceBuffer Rb, Ub, r_ast, M_tmp, res_tmp, cdev;
-   TNLB_TRY_STATUS(Rb.alloc(sizeof(Real) * ld * (ell + 1)));
-   TNLB_TRY_STATUS(Ub.alloc(sizeof(Real) * ld * (ell + 1)));
-   for (auto* q : {&r_ast, &M_tmp, &res_tmp}) TNLB_TRY_STATUS(q->alloc(sizeof(Real) * n));
-   TNLB_TRY_STATUS(cdev.alloc(sizeof(double) * 128));
+   TNLB_TRY_STATUS(Rb.alloc(sizeof(Real) * ld * (ell + 1), c.st));
+   TNLB_TRY_STATUS(Ub.alloc(sizeof(Real) * ld * (ell + 1), c.st));
+   for (auto* q : {&r_ast, &M_tmp, &res_tmp}) TNLB_TRY_STATUS(q->alloc(sizeof(Real) * n, c.st));
+   TNLB_TRY_STATUS(cdev.alloc(sizeof(double) * 128, c.st));
    Real* R = Rb.as<Real>();
    Real* U = Ub.as<Real>();
    auto Rc = [&](int j) { return R + (int64_t)j * ld; };
@@ -1894,12 +1894,12 @@ tnlb_status idrs_solve(const Ctx<Real>& c, const Precond<Real>& Pc, const tnlb_s
    const bool smoothing = prm.idr_residual_smoothing != 0;
    const int64_t ld = (n + 31) / 32 * 32;
    Work W;
-   TNLB_TRY_STATUS(W.alloc());
+   TNLB_TRY_STATUS(W.alloc(c.st));
    DeviceBuffer Pb, Gb, Ub, r, v, pv, t, x_s, r_s, cdev, hdev;
-   for (auto* q : {&Pb, &Gb, &Ub}) TNLB_TRY_STATUS(q->alloc(sizeof(Real) * ld * s));
-   for (auto* q : {&r, &v, &pv, &t, &x_s, &r_s}) TNLB_TRY_STATUS(q->alloc(sizeof(Real) * n));
-   TNLB_TRY_STATUS(cdev.alloc(sizeof(double) * 128));
-   TNLB_TRY_STATUS(hdev.alloc(sizeof(double) * 128));
+   for (auto* q : {&Pb, &Gb, &Ub}) TNLB_TRY_STATUS(q->alloc(sizeof(Real) * ld * s, c.st));
+   for (auto* q : {&r, &v, &pv, &t, &x_s, &r_s}) TNLB_TRY_STATUS(q->alloc(sizeof(Real) * n, c.st));
+   TNLB_TRY_STATUS(cdev.alloc(sizeof(double) * 128, c.st));
+   TNLB_TRY_STATUS(hdev.alloc(sizeof(double) * 128, c.st));
    Real* Pd = Pb.as<Real>();
    Real* Gd = Gb.as<Real>();
    Real* Ud = Ub.as<Real>();
@@ -2120,8 +2120,8 @@ tnlb_status true_residual(const tnlb_segments* seg, tnlb_real real, const int32_
    const size_t rs = real == TNLB_F64 ? 8 : 4;
    DeviceBuffer ax;
    Work W;
-   TNLB_TRY_STATUS(W.alloc());
-   TNLB_TRY_STATUS(ax.alloc(rs * (n > 0 ? n : 1)));
+   TNLB_TRY_STATUS(W.alloc(st));
+   TNLB_TRY_STATUS(ax.alloc(rs * (n > 0 ? n : 1), st));
    TNLB_TRY_STATUS(spmv_dispatch(seg, real, cols, vals, x, ax.ptr, 1.0, 0.0, st));
    if (real == TNLB_F64)
       k_resid_norms<double><<<vec_grid(n), kRedThreads, 0, st>>>(n, (const double*)b, ax.as<double>(), W.red(),
@@ -2207,10 +2207,10 @@ tnlb_status solve_mixed_cg(const tnlb_segments* seg, const int32_t* cols, const 
 {
    const int64_t n = seg->n;
    DeviceBuffer v32, r64, r32, d32, d64;
-   TNLB_TRY_STATUS(v32.alloc(sizeof(float) * (seg->storage > 0 ? seg->storage : 1)));
-   TNLB_TRY_STATUS(r64.alloc(sizeof(double) * n));
-   TNLB_TRY_STATUS(r32.alloc(sizeof(float) * n));
-   TNLB_TRY_STATUS(d32.alloc(sizeof(float) * n));
+   TNLB_TRY_STATUS(v32.alloc(sizeof(float) * (seg->storage > 0 ? seg->storage : 1), st));
+   TNLB_TRY_STATUS(r64.alloc(sizeof(double) * n, st));
+   TNLB_TRY_STATUS(r32.alloc(sizeof(float) * n, st));
+   TNLB_TRY_STATUS(d32.alloc(sizeof(float) * n, st));
    k_convert<float, double><<<grid_for(seg->storage, 256 * 8), 256, 0, st>>>(seg->storage, vals, v32.as<float>());
    TNLB_CHECK_LAUNCH();
    Ctx<float> c32{seg, TNLB_F32, cols, v32.as<float>(), n, st};
@@ -2229,7 +2229,7 @@ tnlb_status solve_mixed_cg(const tnlb_segments* seg, const int32_t* cols, const 
    *outer = 0;
    double resid = 0;
    Work W;
-   TNLB_TRY_STATUS(W.alloc());
+   TNLB_TRY_STATUS(W.alloc(st));
    for (int o = 0; o <= max_outer; o++) {
       // A x in FP64; the residual norm computed as tnlb_true_residual does
       TNLB_TRY_STATUS(spmv_dispatch(seg, TNLB_F64, cols, vals, x, r64.ptr, 1.0, 0.0, st));
@@ -2851,19 +2851,21 @@ tnlb_status reliable_t(const tnlb_segments* seg, const int32_t* cols, const doub
    // kernels (band.cuh) read whole 16-byte groups
    const int64_t npad = (n + 3) / 4 * 4;
    DeviceBuffer v32, ax, r, z, p, Ap, xc, scal;
-   TNLB_TRY_STATUS(v32.alloc(sizeof(float) * (seg->storage > 0 ? seg->storage : 1)));
-   TNLB_TRY_STATUS(ax.alloc(sizeof(double) * n));
-   TNLB_TRY_STATUS(r.alloc(sizeof(VT) * npad));
-   TNLB_TRY_STATUS(z.alloc(sizeof(VT) * npad));
-   TNLB_TRY_STATUS(p.alloc(sizeof(VT) * npad));
-   TNLB_TRY_STATUS(Ap.alloc(sizeof(VT) * npad));
-   TNLB_TRY_STATUS(xc.alloc(sizeof(double) * npad));  // the correction is FP64 (ru_entry)
-   TNLB_TRY_STATUS(scal.alloc(sizeof(double) * 4));  // [0] (p, Ap), [1] (r, z), [2..3] residual sums
+   TNLB_TRY_STATUS(v32.alloc(sizeof(float) * (seg->storage > 0 ? seg->storage : 1), st));
+   TNLB_TRY_STATUS(ax.alloc(sizeof(double) * n, st));
+   TNLB_TRY_STATUS(r.alloc(sizeof(VT) * npad, st));
+   TNLB_TRY_STATUS(z.alloc(sizeof(VT) * npad, st));
+   TNLB_TRY_STATUS(p.alloc(sizeof(VT) * npad, st));
+   TNLB_TRY_STATUS(Ap.alloc(sizeof(VT) * npad, st));
+   TNLB_TRY_STATUS(xc.alloc(sizeof(double) * npad, st));  // the correction is FP64 (ru_entry)
+   TNLB_TRY_STATUS(scal.alloc(sizeof(double) * 4, st));  // [0] (p, Ap), [1] (r, z), [2..3] residual sums
    k_convert<float, double><<<grid_for(seg->storage, 256 * 8), 256, 0, st>>>(seg->storage, vals, v32.as<float>());
    TNLB_CHECK_LAUNCH();
    tnlb_precond* own = nullptr;
-   if (!inner_precond && inner_kind != TNLB_PRECOND_NONE)
+   if (!inner_precond && inner_kind != TNLB_PRECOND_NONE) {
+      PoolScope scope(st);  // destroyed at the end of this call
       TNLB_TRY_STATUS(precond_create(inner_kind, seg, TNLB_F32, cols, v32.ptr, st, &own));
+   }
    struct Guard {
       tnlb_precond* p;
       ~Guard() { delete p; }
@@ -2883,10 +2885,10 @@ tnlb_status reliable_t(const tnlb_segments* seg, const int32_t* cols, const doub
    TNLB_REQUIRE(mode != 2 || fused_m || kVec == TNLB_F32, TNLB_ERR_INVALID_ARGUMENT,
                 "solve_mixed_reliable: FP64 vectors need an FSAI whose factors hold at most 16 entries per row");
    Work W;  // reductions of the vector kernels
-   TNLB_TRY_STATUS(W.alloc());
+   TNLB_TRY_STATUS(W.alloc(st));
    Work WA, WM;  // reductions of the fused products
-   TNLB_TRY_STATUS(WA.alloc());
-   TNLB_TRY_STATUS(WM.alloc());
+   TNLB_TRY_STATUS(WA.alloc(st));
+   TNLB_TRY_STATUS(WM.alloc(st));
    RuState* S = reinterpret_cast<RuState*>(W.S());
    static_assert(sizeof(RuState) <= sizeof(DevState), "RuState must fit the state buffer");
    double* pap = scal.as<double>();
@@ -2908,6 +2910,7 @@ tnlb_status reliable_t(const tnlb_segments* seg, const int32_t* cols, const doub
    CompactCopy cA, cG, cGT;
    const bool compact_dia = prm.reliable_layout != 1;
    if (kVec == TNLB_F32) {
+      PoolScope scope(st);
       if (fused_a)
          TNLB_TRY_STATUS(compact_build(seg, cols, v32f, false, 1.0f, compact_dia, st, &cA,
                                        prm.reliable_operator == 0 ? vals : nullptr));
@@ -2943,8 +2946,8 @@ tnlb_status reliable_t(const tnlb_segments* seg, const int32_t* cols, const doub
    const bool fused_u = cmp_m;
    DeviceBuffer r2, tb;
    if (fused_u) {
-      TNLB_TRY_STATUS(r2.alloc(sizeof(float) * npad));
-      TNLB_TRY_STATUS(tb.alloc(sizeof(float) * npad));
+      TNLB_TRY_STATUS(r2.alloc(sizeof(float) * npad, st));
+      TNLB_TRY_STATUS(tb.alloc(sizeof(float) * npad, st));
    }
    float* tvec = fused_u ? tb.as<float>() : mode == 2 ? (float*)fsai_view(pobj->fsai).tmp : nullptr;
    TNLB_REQUIRE(!fused_u || aligned16(tvec), TNLB_ERR_INVALID_ARGUMENT,
@@ -3098,7 +3101,7 @@ tnlb_status reliable_t(const tnlb_segments* seg, const int32_t* cols, const doub
    // true residual so far (xbest).
    constexpr int32_t kStallWindow = 16384;
    DeviceBuffer xbest;
-   TNLB_TRY_STATUS(xbest.alloc(sizeof(double) * n));
+   TNLB_TRY_STATUS(xbest.alloc(sizeof(double) * n, cs));
    double best = HUGE_VAL, lowest = HUGE_VAL;
    int32_t it_best = 0;
    bool stalled = false;

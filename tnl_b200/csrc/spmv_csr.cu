@@ -832,7 +832,7 @@ tnlb_status build_csr_tile_plan(tnlb_segments* seg, cudaStream_t stream)
    TNLB_CHECK_LAUNCH();
    // longest row, for the choice of the default kernel
    DeviceBuffer mx;
-   TNLB_TRY_STATUS(mx.alloc(sizeof(int32_t)));
+   TNLB_TRY_STATUS(mx.alloc(sizeof(int32_t), stream));
    TNLB_CUDA_TRY(cudaMemsetAsync(mx.ptr, 0, sizeof(int32_t), stream));
    if (seg->n > 0) {
       k_max_row<<<grid_for(seg->n, 256 * 8), 256, 0, stream>>>(seg->offsets.as<int32_t>(), seg->n, mx.as<int32_t>());
