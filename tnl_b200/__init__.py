@@ -279,10 +279,16 @@ class SparseMatrix:
         caps = _device_i32(capacities)
         if caps.numel() != self.rows:
             raise ValueError("setRowCapacities: the number of capacities does not match the number of rows")
-        self.segments.setSegmentsSizes(caps)
+        self._allocate(caps)
+        self.values.zero_()
+        self.columnIndexes.fill_(-1)
+
+    def _allocate(self, capacities: torch.Tensor) -> None:
+        """Segments of the given capacities and their slots, uninitialised."""
+        self.segments.setSegmentsSizes(capacities)
         st = self.segments.getStorageSize()
-        self.values = torch.zeros(st, dtype=self.real, device="cuda")
-        self.columnIndexes = torch.full((st,), -1, dtype=torch.int32, device="cuda")
+        self.values = torch.empty(st, dtype=self.real, device="cuda")
+        self.columnIndexes = torch.empty(st, dtype=torch.int32, device="cuda")
 
     def assign(self, rowptr, cols, vals, columns: int | None = None) -> "SparseMatrix":
         """Cross-format ``operator=`` from a CSR matrix (SparseOperations.hpp:106-186).
@@ -296,7 +302,7 @@ class SparseMatrix:
         v = (vals if isinstance(vals, torch.Tensor) else torch.as_tensor(np.ascontiguousarray(vals)))
         v = v.to(device="cuda", dtype=self.real).contiguous()
         self.setDimensions(n, n if columns is None else columns)
-        self.setRowCapacities(rp[1:] - rp[:-1])
+        self._allocate(rp[1:] - rp[:-1])  # the fill writes every slot
         check(capi.tnlb_matrix_fill_from_csr(self.segments.handle, _real_code(self.real), rp.data_ptr(),
                                              c.data_ptr() if c.numel() else None, v.data_ptr() if v.numel() else None,
                                              self.columnIndexes.data_ptr() if self.columnIndexes.numel() else None,
