@@ -247,7 +247,7 @@ tnlb_status tnlb_spmv(const tnlb_segments* seg, tnlb_real real, const int32_t* d
    else {
       TNLB_REQUIRE(kernel == TNLB_KERNEL_DEFAULT || kernel == TNLB_KERNEL_VECTOR || kernel == TNLB_KERNEL_SCALAR,
                    TNLB_ERR_INVALID_ARGUMENT, "kernel not available for this format");
-      s = spmv_ell_family(seg, real, d_cols, d_values, d_x, d_y, alpha, beta, begin, end, kernel,
+      s = spmv_ell_family(seg, real, d_cols, d_values, columns, d_x, d_y, alpha, beta, begin, end, kernel,
                           kernel == TNLB_KERNEL_SCALAR ? 1 : threads_per_segment, (cudaStream_t)stream, &launches);
    }
    g_last_launches = launches;

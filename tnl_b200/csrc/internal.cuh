@@ -391,8 +391,9 @@ tnlb_status spmv_xpby(const tnlb_segments* seg, tnlb_real real, const int32_t* c
 tnlb_status spmv_csr(const tnlb_segments* seg, tnlb_real real, const int32_t* cols, const void* vals, const void* x,
                      void* y, double alpha, double beta, int32_t begin, int32_t end, tnlb_kernel kernel, int32_t tps,
                      cudaStream_t stream, int* launches, const int32_t* skip = nullptr);
+// x holds `columns` entries.
 tnlb_status spmv_ell_family(const tnlb_segments* seg, tnlb_real real, const int32_t* cols, const void* vals,
-                            const void* x, void* y, double alpha, double beta, int32_t begin, int32_t end,
+                            int32_t columns, const void* x, void* y, double alpha, double beta, int32_t begin, int32_t end,
                             tnlb_kernel kernel, int32_t tps, cudaStream_t stream, int* launches);
 tnlb_status build_csr_tile_plan(tnlb_segments* seg, cudaStream_t stream);
 // solvers.cu / ilu0.cu / fsai.cu

@@ -492,7 +492,8 @@ tnlb_status spmv_dispatch(const tnlb_segments* seg, tnlb_real real, const int32_
       return spmv_csr(seg, real, cols, vals, x, y, alpha, beta, 0, seg->n,
                       seg->format == TNLB_ADAPTIVE_CSR ? TNLB_KERNEL_ADAPTIVE : TNLB_KERNEL_DEFAULT, 0, st, &launches,
                       seg->format == TNLB_CSR ? skip : nullptr);
-   return spmv_ell_family(seg, real, cols, vals, x, y, alpha, beta, 0, seg->n, TNLB_KERNEL_DEFAULT, 0, st, &launches);
+   return spmv_ell_family(seg, real, cols, vals, seg->n, x, y, alpha, beta, 0, seg->n, TNLB_KERNEL_DEFAULT, 0, st,
+                          &launches);
 }
 
 namespace {
