@@ -643,8 +643,8 @@ constexpr int32_t kPersistCap = 2048;
 
 // Runs a resident solver kernel (persist.cuh) until the state is done and reads
 // it back.  `args`: the kernel's arguments up to n.
-tnlb_status persist_run(const void* kern, const PersistShape& sh, std::vector<void*> args, int32_t n, const Work& W,
-                        cudaStream_t st, DevState* h)
+tnlb_status persist_run(const PersistShape& sh, std::vector<void*> args, int32_t n, const Work& W, cudaStream_t st,
+                        DevState* h)
 {
    DeviceBuffer sync;
    TNLB_TRY_STATUS(sync.alloc(kPersistSlotBytes + sizeof(int32_t), st));
@@ -654,7 +654,7 @@ tnlb_status persist_run(const void* kern, const PersistShape& sh, std::vector<vo
    for (void* a : {(void*)&n, (void*)&S, (void*)&g, (void*)&cap}) args.push_back(a);
    do {
       TNLB_CUDA_TRY(cudaMemsetAsync(sync.ptr, 0, sync.bytes, st));
-      TNLB_CUDA_TRY(cudaLaunchCooperativeKernel(kern, dim3(sh.blocks), dim3(sh.threads), args.data(), sh.smem, st));
+      TNLB_CUDA_TRY(persist_launch(sh, args.data(), st));
       TNLB_CUDA_TRY(cudaMemcpyAsync(h, S, sizeof(*h), cudaMemcpyDeviceToHost, st));
       TNLB_CUDA_TRY(cudaMemcpyAsync(&err, g.err, sizeof(err), cudaMemcpyDeviceToHost, st));
       TNLB_CUDA_TRY(cudaStreamSynchronize(st));
@@ -710,13 +710,12 @@ tnlb_status cg_solve(const Ctx<Real>& c, const Precond<Real>& P, const tnlb_solv
    else
       k_cg_init<Real><<<G, kRedThreads, 0, c.st>>>(n, r.as<Real>(), z.as<Real>(), p.as<Real>(), P.d(), W.red(), W.S());
    TNLB_CHECK_LAUNCH();
-   const void* kern = persist_rows_fit(c.seg) && !gen ? persist_pick<Real, CgPersistKernel>(c.seg) : nullptr;
-   PersistShape sh;
-   if (kern && persist_shape(kern, (int32_t)n, 4, sizeof(Real), sh)) {
+   const PersistShape sh = gen ? PersistShape{} : persist_cg<Real>(c.seg);
+   if (sh.kernel) {
       PersistVectors<Real, 4> V{{Ap.as<Real>(), r.as<Real>(), x, const_cast<Real*>(P.d())}, sh.kept, sh.rows};
       PersistRows<Real> A = persist_rows(c.seg, c.cols, c.vals);
       Real* pp = p.as<Real>();
-      TNLB_TRY_STATUS(persist_run(kern, sh, {&A, &V, &pp}, (int32_t)n, W, c.st, &h));
+      TNLB_TRY_STATUS(persist_run(sh, {&A, &V, &pp}, (int32_t)n, W, c.st, &h));
       res->iterations = h.it;
       res->residue = h.residue;
       res->converged = check_convergence(h.residue, h.it, h.maxit, h.minit, h.conv, h.div);
@@ -995,11 +994,9 @@ tnlb_status bicgstab_solve(const Ctx<Real>& c, const Precond<Real>& P, const tnl
       return TNLB_OK;
    };
    const bool diagonal = P.kind == TNLB_PRECOND_NONE || P.kind == TNLB_PRECOND_JACOBI;
-   const void* kern = diagonal && !prm.bicgstab_exact_residue && persist_rows_fit(c.seg)
-                         ? persist_pick<Real, BicgPersistKernel>(c.seg)
-                         : nullptr;
-   PersistShape sh;
-   const bool persist = kern && persist_shape(kern, (int32_t)n, 6, sizeof(Real), sh);
+   const PersistShape sh =
+      diagonal && !prm.bicgstab_exact_residue ? persist_bicgstab<Real>(c.seg) : PersistShape{};
+   const bool persist = sh.kernel != nullptr;
    if (persist) {
       PersistVectors<Real, 6> V{{Ap.as<Real>(), r.as<Real>(), As.as<Real>(), r_ast.as<Real>(), x,
                                  const_cast<Real*>(P.d())},
@@ -1015,7 +1012,7 @@ tnlb_status bicgstab_solve(const Ctx<Real>& c, const Precond<Real>& P, const tnl
       while (h.done != 1) {
          h.done = 0;
          TNLB_CUDA_TRY(cudaMemcpyAsync(W.S(), &h, sizeof(h), cudaMemcpyHostToDevice, c.st));
-         TNLB_TRY_STATUS(persist_run(kern, sh, {&A, &V, &pp, &ps}, (int32_t)n, W, c.st, &h));
+         TNLB_TRY_STATUS(persist_run(sh, {&A, &V, &pp, &ps}, (int32_t)n, W, c.st, &h));
          if (h.done != kPersistRestart) continue;
          TNLB_TRY_STATUS(restart());
          h.beta = (rho / h.rho_old) * (h.alpha / h.omega);
