@@ -1,5 +1,5 @@
-// persist.cuh -- CG and BiCGStab iterations in one resident kernel (persist.cu):
-// what the solvers need to launch them.
+// persist.cuh -- CG and BiCGStab iterations and Gram-Schmidt in one resident
+// kernel (persist.cu): what the solvers need to launch them.
 #pragma once
 
 #include "internal.cuh"
@@ -96,6 +96,10 @@ template <typename Real>
 PersistShape persist_cg(const tnlb_segments* seg);
 template <typename Real>
 PersistShape persist_bicgstab(const tnlb_segments* seg);
+// Gram-Schmidt: also null where a block's rows of three vectors do not fit its
+// shared memory (1.3M rows in FP64).
+template <typename Real>
+PersistShape persist_mgs(int64_t n);
 cudaError_t persist_launch(const PersistShape& sh, void** args, cudaStream_t st);
 
 }  // namespace tnlb

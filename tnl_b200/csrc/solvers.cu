@@ -1360,6 +1360,16 @@ tnlb_status gmres_solve(const Ctx<Real>& c, const Precond<Real>& P, const tnlb_s
    if (flexible) TNLB_TRY_STATUS(Z.alloc(sizeof(Real) * ld * m_max, c.st));
    Real* Vp = V.as<Real>();
    double* sc = W.scratch.as<double>();
+   // MGS in one resident kernel an Arnoldi step (persist.cuh) while a block's
+   // rows of w and of two columns fit its shared memory (1.3M rows in FP64)
+   PersistShape mgs_shape;
+   if (variant == TNLB_GMRES_MGS || variant == TNLB_GMRES_MGSR) mgs_shape = persist_mgs<Real>(n);
+   const bool mgs_resident = mgs_shape.kernel != nullptr;
+   DeviceBuffer mgs_sync;
+   TNLB_TRY_STATUS(mgs_sync.alloc(kPersistSlotBytes + sizeof(int32_t), c.st));
+   TNLB_CUDA_TRY(cudaMemsetAsync(mgs_sync.ptr, 0, mgs_sync.bytes, c.st));
+   PersistSync mgs_g = persist_sync(mgs_sync);
+   int64_t ld_v = ld;
    const unsigned G = vec_grid(n);
    const bool pre = P.kind != TNLB_PRECOND_NONE && !flexible;
    const bool rightp = P.kind != TNLB_PRECOND_NONE && flexible;
@@ -1487,6 +1497,24 @@ tnlb_status gmres_solve(const Ctx<Real>& c, const Precond<Real>& P, const tnlb_s
             }
             normw = hs[0];
          }
+         else if (mgs_resident) {
+            double* hd = hdev.as<double>();
+            Real* wp = w.as<Real>();
+            int32_t cols = i + 1, passes = reorth, n32 = (int32_t)n;
+            TNLB_CUDA_TRY(cudaMemsetAsync(mgs_sync.ptr, 0, kPersistSlotBytes, c.st));
+            void* args[] = {&Vp, &ld_v, &wp, &cols, &passes, &mgs_shape.rows, &n32, &hd, &sc, &mgs_g};
+            TNLB_CUDA_TRY(persist_launch(mgs_shape, args, c.st));
+            std::vector<double> hall(2 * 64);
+            int32_t err = 0;
+            TNLB_CUDA_TRY(cudaMemcpyAsync(hall.data(), hd, sizeof(double) * 2 * 64, cudaMemcpyDeviceToHost, c.st));
+            TNLB_CUDA_TRY(cudaMemcpyAsync(hs, sc, sizeof(double), cudaMemcpyDeviceToHost, c.st));
+            TNLB_CUDA_TRY(cudaMemcpyAsync(&err, mgs_g.err, sizeof(err), cudaMemcpyDeviceToHost, c.st));
+            TNLB_CUDA_TRY(cudaStreamSynchronize(c.st));
+            TNLB_REQUIRE(err == 0, TNLB_ERR_CUDA, "solver kernel: a wait between blocks ran out");
+            for (int l = 0; l < reorth; l++)
+               for (int k = 0; k <= i; k++) H[k + i * (m + 1)] += hall[l * 64 + k];
+            normw = hs[0];
+         }
          else {
             // MGS: H_{k,i} = (w, v_k); w -= H_{k,i} v_k for k = 0..i, `reorth`
             // passes.  Each kernel applies one update and computes the next
@@ -1515,9 +1543,11 @@ tnlb_status gmres_solve(const Ctx<Real>& c, const Precond<Real>& P, const tnlb_s
             normw = hs[0];
          }
          H[i + 1 + i * (m + 1)] = normw;
-         k_scale<Real><<<vec_grid(n), kRedThreads, 0, c.st>>>(n, (Real)(1.0 / normw), w.as<Real>(),
-                                                              Vp + (int64_t)(i + 1) * ld);
-         TNLB_CHECK_LAUNCH();
+         if (!mgs_resident) {
+            k_scale<Real><<<vec_grid(n), kRedThreads, 0, c.st>>>(n, (Real)(1.0 / normw), w.as<Real>(),
+                                                                 Vp + (int64_t)(i + 1) * ld);
+            TNLB_CHECK_LAUNCH();
+         }
          // Givens rotations (GMRES.hpp:731-770)
          for (int k = 0; k < i; k++) rot_apply(H[k + i * (m + 1)], H[k + 1 + i * (m + 1)], cs[k], sn[k]);
          if (H[i + 1 + i * (m + 1)] != 0.0) {
