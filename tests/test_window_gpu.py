@@ -1,4 +1,4 @@
-"""Products that keep a window of x in shared memory, against numpy in
+"""Products that keep a window of x or y in shared memory, against numpy in
 FP64.
 
 Matrices at the rules' edges: columns inside the window, half outside, all
@@ -24,7 +24,7 @@ SHAPES = {  # rows, columns, half band (None: anywhere)
 def _matrix(rows, columns, half, longest, seed, triangle=False):
     rng = np.random.default_rng(seed)
     lens = rng.integers(0, longest + 1, rows)
-    lens[rows // 2] = 3 * longest
+    lens[rows // 2] = longest + 20
     rp = np.zeros(rows + 1, np.int32)
     np.cumsum(lens, out=rp[1:])
     row = np.repeat(np.arange(rows), lens)
@@ -50,7 +50,7 @@ def _vectors(real, columns, rows):
 
 @pytest.mark.parametrize("real", ["float64", "float32"])
 @pytest.mark.parametrize("shape", SHAPES)
-@pytest.mark.parametrize("fmt", ["SlicedEllpack"])
+@pytest.mark.parametrize("fmt", ["SlicedEllpack", "CSR"])
 def test_products_of_long_rows(fmt, shape, real):
     import tnl_b200 as t
 
@@ -65,4 +65,34 @@ def test_products_of_long_rows(fmt, shape, real):
     prod = vals * x[cols]
     want = 0.5 * y0 - 1.5 * np.bincount(row, prod, minlength=rows)
     scale = np.abs(0.5 * y0) + 1.5 * np.bincount(row, np.abs(prod), minlength=rows)
+    _close(out, want, scale, real)
+    # transposed, into a part of the columns
+    out = xs.clone()
+    first, last = columns // 7, columns - 11
+    M.transposedVectorProduct(ys, out, 2.0, 0.5, first, last)
+    prod = vals * y0[row]
+    inside = (np.arange(columns) >= first) & (np.arange(columns) < last)
+    want = 0.5 * x + 2.0 * np.where(inside, np.bincount(cols, prod, minlength=columns), 0.0)
+    scale = np.abs(0.5 * x) + 2.0 * np.bincount(cols, np.abs(prod), minlength=columns)
+    _close(out, want, scale, real)
+
+
+@pytest.mark.parametrize("real", ["float64", "float32"])
+@pytest.mark.parametrize("half,longest", [(300, 3), (300, 20), (9000, 24), (None, 20)])
+@pytest.mark.parametrize("fmt", ["SlicedEllpack", "CSR", "Ellpack"])
+def test_symmetric_product(fmt, half, longest, real):
+    import tnl_b200 as t
+
+    n = 130001
+    rp, cols, vals, row = _matrix(n, n, half, longest, 4, triangle=True)
+    vals = vals.astype(real).astype(np.float64)
+    M = t.SparseMatrix(t.FORMATS[fmt], getattr(torch, real), symmetric=True).assign(rp, cols, vals, n)
+    x, y0 = _vectors(real, n, n)
+    xs, out = (torch.tensor(v, dtype=getattr(torch, real), device="cuda") for v in (x, y0))
+    M.vectorProduct(xs, out, 1.5, -1.0)
+    low = cols < row
+    want, scale = -y0, np.abs(y0)
+    for r, c, v in ((row, cols, vals), (cols[low], row[low], vals[low])):
+        want = want + 1.5 * np.bincount(r, v * x[c], minlength=n)
+        scale = scale + 1.5 * np.bincount(r, np.abs(v * x[c]), minlength=n)
     _close(out, want, scale, real)
