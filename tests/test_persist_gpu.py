@@ -146,3 +146,42 @@ def test_resident_cg_over_several_launches():
     S.solve(b, x)
     assert S.getIterations() == 2102
     assert abs(t.true_residual(mat, b, x) / S.getResidue() - 1) < 1e-3
+
+
+@pytest.mark.parametrize("real", ["float64", "float32"])
+@pytest.mark.parametrize("variant", ["MGS", "MGSR"])
+@pytest.mark.parametrize("n", [33, 20000, 20001, 151553])
+def test_resident_gram_schmidt_matches_numpy(n, variant, real):
+    """Seven GMRES iterations across a restart of 4: one cluster, the grid."""
+    import tnl_b200 as t
+
+    rp, cols, vals, rows = _matrix(n, (1, 5), False, n)
+    dtype = getattr(torch, real)
+    vals = vals.astype(real).astype(np.float64)
+    b = np.random.default_rng(1).uniform(-1, 1, n).astype(real).astype(np.float64)
+    x = np.zeros(n)
+    for steps in (4, 3):
+        r = b - np.bincount(rows, vals * x[cols], minlength=n)
+        V, H = [r / np.linalg.norm(r)], np.zeros((steps + 1, steps))
+        for i in range(steps):
+            w = np.bincount(rows, vals * V[i][cols], minlength=n)
+            for _ in range(2):
+                for k in range(i + 1):
+                    h = w @ V[k]
+                    H[k, i] += h
+                    w = w - h * V[k]
+            H[i + 1, i] = np.linalg.norm(w)
+            V.append(w / H[i + 1, i])
+        e = np.zeros(steps + 1)
+        e[0] = np.linalg.norm(r)
+        x = x + np.linalg.lstsq(H, e, rcond=None)[0] @ np.array(V[:steps])
+    mat = t.SparseMatrix(t.CSR, dtype).assign(rp, cols, vals)
+    S = t.GMRES()
+    S.setMatrix(mat)
+    S.setConvergenceResidue(0.0)
+    S.setMaxIterations(6)
+    S.setup({"gmres-variant": variant, "gmres-restarting-min": 4, "gmres-restarting-max": 4})
+    y = torch.zeros(n, dtype=dtype, device="cuda")
+    S.solve(torch.tensor(b, dtype=dtype, device="cuda"), y)
+    err = np.linalg.norm(y.cpu().numpy().astype(np.float64) - x)
+    assert err <= (1e-13 if real == "float64" else 2e-5) * np.linalg.norm(x)

@@ -7,11 +7,12 @@
 // returns checkConvergence()).  What changes is where the scalars live: every
 // dot product and norm is reduced on the device into a DevState record, and
 // the scalar recurrences (alpha, beta, residue, the stopping test) run in the
-// last block of the reduction.  CG never waits for the host inside an
-// iteration: batches of iterations are captured once in a CUDA graph and
-// replayed; kernels of iterations past the stopping point return at once on
-// the device `done` flag, so the iteration count is exact.  BiCGStab and
-// GMRES read the state once per iteration / Arnoldi step.  GMRES keeps the
+// last block of the reduction.  CG and BiCGStab on short rows, with Jacobi or no
+// preconditioner, run in one resident kernel (persist.cu).  Otherwise CG's
+// iterations are captured in batches in a CUDA graph and replayed; kernels of
+// iterations past the stopping point return at once on the device `done` flag, so
+// the iteration count is exact; BiCGStab reads the state every iteration, and
+// GMRES every Arnoldi step.  GMRES keeps the
 // small Hessenberg least-squares problem (Givens rotations, back
 // substitution) on the host in FP64, as the reference does.
 #include <cfloat>
@@ -1366,9 +1367,11 @@ tnlb_status gmres_solve(const Ctx<Real>& c, const Precond<Real>& P, const tnlb_s
    if (variant == TNLB_GMRES_MGS || variant == TNLB_GMRES_MGSR) mgs_shape = persist_mgs<Real>(n);
    const bool mgs_resident = mgs_shape.kernel != nullptr;
    DeviceBuffer mgs_sync;
-   TNLB_TRY_STATUS(mgs_sync.alloc(kPersistSlotBytes + sizeof(int32_t), c.st));
+   constexpr size_t kMgsWords = 2 * 64 + 2;  // the dot products, |w|, the error flag
+   TNLB_TRY_STATUS(mgs_sync.alloc(kPersistSlotBytes + sizeof(double) * kMgsWords, c.st));
    TNLB_CUDA_TRY(cudaMemsetAsync(mgs_sync.ptr, 0, mgs_sync.bytes, c.st));
-   PersistSync mgs_g = persist_sync(mgs_sync);
+   double* mgs_h = reinterpret_cast<double*>(mgs_sync.as<unsigned char>() + kPersistSlotBytes);
+   PersistSync mgs_g{mgs_sync.as<ulonglong2>(), reinterpret_cast<int32_t*>(mgs_h + 2 * 64 + 1)};
    int64_t ld_v = ld;
    const unsigned G = vec_grid(n);
    const bool pre = P.kind != TNLB_PRECOND_NONE && !flexible;
@@ -1498,22 +1501,19 @@ tnlb_status gmres_solve(const Ctx<Real>& c, const Precond<Real>& P, const tnlb_s
             normw = hs[0];
          }
          else if (mgs_resident) {
-            double* hd = hdev.as<double>();
+            double *hd = mgs_h, *normp = mgs_h + 2 * 64;
             Real* wp = w.as<Real>();
             int32_t cols = i + 1, passes = reorth, n32 = (int32_t)n;
             TNLB_CUDA_TRY(cudaMemsetAsync(mgs_sync.ptr, 0, kPersistSlotBytes, c.st));
-            void* args[] = {&Vp, &ld_v, &wp, &cols, &passes, &mgs_shape.rows, &n32, &hd, &sc, &mgs_g};
+            void* args[] = {&Vp, &ld_v, &wp, &cols, &passes, &mgs_shape.rows, &n32, &hd, &normp, &mgs_g};
             TNLB_CUDA_TRY(persist_launch(mgs_shape, args, c.st));
-            std::vector<double> hall(2 * 64);
-            int32_t err = 0;
-            TNLB_CUDA_TRY(cudaMemcpyAsync(hall.data(), hd, sizeof(double) * 2 * 64, cudaMemcpyDeviceToHost, c.st));
-            TNLB_CUDA_TRY(cudaMemcpyAsync(hs, sc, sizeof(double), cudaMemcpyDeviceToHost, c.st));
-            TNLB_CUDA_TRY(cudaMemcpyAsync(&err, mgs_g.err, sizeof(err), cudaMemcpyDeviceToHost, c.st));
+            double hall[kMgsWords];
+            TNLB_CUDA_TRY(cudaMemcpyAsync(hall, hd, sizeof(hall), cudaMemcpyDeviceToHost, c.st));
             TNLB_CUDA_TRY(cudaStreamSynchronize(c.st));
-            TNLB_REQUIRE(err == 0, TNLB_ERR_CUDA, "solver kernel: a wait between blocks ran out");
+            TNLB_REQUIRE(hall[2 * 64 + 1] == 0, TNLB_ERR_CUDA, "solver kernel: a wait between blocks ran out");
             for (int l = 0; l < reorth; l++)
                for (int k = 0; k <= i; k++) H[k + i * (m + 1)] += hall[l * 64 + k];
-            normw = hs[0];
+            normw = hall[2 * 64];
          }
          else {
             // MGS: H_{k,i} = (w, v_k); w -= H_{k,i} v_k for k = 0..i, `reorth`
