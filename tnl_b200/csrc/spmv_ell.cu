@@ -102,15 +102,48 @@ __global__ void k_ell_row(const int32_t* __restrict__ cols, const Real* __restri
 
 // ------------------------------------------------------- SlicedEllpack
 
-// G warps per slice (G = 1, 2, 4, 8); the block holds 8/G slices.
+// The runs of slices that k_sell_window takes, and the window of each: `room`
+// entries of x around the run's rows.
+struct SellWindow {
+   int32_t per_block, columns, room;  // slices of a run, a multiple of 8; 0: no windows
+   __device__ __forceinline__ int32_t lo(int64_t s0, int64_t s1) const
+   {
+      const int64_t mid = (s0 + s1) / 2 * kSellSlice;
+      return (int32_t)imin64(imax64(mid - room / 2, 0), imax64((int64_t)columns - room, 0));
+   }
+   __device__ __forceinline__ uint32_t width(int32_t lo) const { return (uint32_t)imin64(room, columns - lo); }
+   // Whether most columns of run `b` lie in its window, from 32 slots of 8 of its
+   // slices.  Called by whole blocks of at least 256 threads; the answer is the
+   // same in each.
+   __device__ __forceinline__ bool taken(int32_t b, const int32_t* cols, const int32_t* slice_off,
+                                         const int32_t* slice_w, int32_t slices) const
+   {
+      const int64_t s0 = (int64_t)b * per_block, s1 = imin64(s0 + per_block, slices);
+      const int32_t l = lo(s0, s1);
+      int32_t c = -1;
+      if (threadIdx.x < 256) {
+         const int64_t s = s0 + (threadIdx.x >> 5) * (s1 - s0) / 8;
+         const int32_t w = slice_w[s];
+         if (w > 0) c = cols[(int64_t)slice_off[s] + (int64_t)(w - 1) / 2 * kSellSlice + (threadIdx.x & 31)];
+      }
+      const int valid = __syncthreads_count(c >= 0);
+      return 2 * __syncthreads_count(c >= 0 && (uint32_t)(c - l) < width(l)) >= valid;
+   }
+};
+
+// G warps per slice (G = 1, 2, 4, 8); the block holds 8/G slices.  Runs that
+// k_sell_window takes are left out.
 template <typename Real, int G>
 __global__ void __launch_bounds__(256) k_sell_col(const int32_t* __restrict__ cols, const Real* __restrict__ vals,
                                                   const Real* __restrict__ x, Real* __restrict__ y,
                                                   const int32_t* __restrict__ slice_off,
                                                   const int32_t* __restrict__ slice_w, int32_t slices, int32_t begin,
-                                                  int32_t end, Real alpha, Real beta)
+                                                  int32_t end, Real alpha, Real beta, SellWindow win)
 {
    __shared__ Real part[8][32];
+   if (win.per_block > 0 &&
+       win.taken((int32_t)((int64_t)blockIdx.x * (8 / G) / win.per_block), cols, slice_off, slice_w, slices))
+      return;
    const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
    const int sub = wib % G;
    const int64_t slice = (int64_t)blockIdx.x * (8 / G) + wib / G;
@@ -233,8 +266,10 @@ __global__ void __launch_bounds__(256) k_sell_walk(const int32_t* __restrict__ c
 // slices keeps the x of its rows and of the columns around them in shared
 // memory.  Columns that differ from lane to lane take the L1 cache one lookup a
 // lane (27M of them, 96 us at one a cycle and SM), shared memory about 3.5
-// cycles for 32.  Nothing is known of the columns beforehand, so the block first
-// looks at some of its slots and gathers from memory where most lie outside.
+// cycles for 32.  Nothing is known of the columns beforehand, so a block first
+// looks at some of its slots and leaves its run to k_sell_col, launched after it,
+// where most lie outside: gathers from memory want the L1 that the window takes,
+// 143 against 73 us for random columns at 500,000 rows (FP64).
 // FP32 residual at 1,000,003 rows of 9 to 45 entries in a band of 20,000: 102.6
 // us by two warps a slice, 82.4 so; its 370 MB with the padding take 57.
 constexpr int kWindowThreads = 1024, kWindowWarps = kWindowThreads / 32, kWindowDepth = 8;
@@ -244,33 +279,23 @@ template <typename Real>
 __global__ void __launch_bounds__(kWindowThreads, 1)
    k_sell_window(const int32_t* __restrict__ cols, const Real* __restrict__ vals, const Real* __restrict__ x,
                  Real* __restrict__ y, const int32_t* __restrict__ slice_off, const int32_t* __restrict__ slice_w,
-                 int32_t slices, int32_t per_block, int32_t columns, int32_t room, int32_t begin, int32_t end,
-                 Real alpha, Real beta)
+                 int32_t slices, SellWindow sw, int32_t begin, int32_t end, Real alpha, Real beta)
 {
    Real* win = reinterpret_cast<Real*>(window_smem);
    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-   const int32_t s0 = (int32_t)imin64((int64_t)blockIdx.x * per_block, slices);
-   const int32_t s1 = (int32_t)imin64((int64_t)s0 + per_block, slices);
-   // the window: `room` entries around the rows' middle
-   const int64_t mid = ((int64_t)s0 + s1) / 2 * kSellSlice;
-   const int32_t lo = (int32_t)imin64(imax64(mid - room / 2, 0), imax64((int64_t)columns - room, 0));
-   const uint32_t width = (uint32_t)imin64(room, columns - lo);
+   if (!sw.taken(blockIdx.x, cols, slice_off, slice_w, slices)) return;
+   const int32_t s0 = (int32_t)blockIdx.x * sw.per_block;
+   const int32_t s1 = (int32_t)imin64((int64_t)s0 + sw.per_block, slices);
+   const int32_t lo = sw.lo(s0, s1);
+   const uint32_t width = sw.width(lo);
    int32_t s = s0 + warp;
    int32_t o = 0, w = 0;
    if (s < s1) {
       o = slice_off[s];
       w = slice_w[s];
    }
-   int c0 = w > 0 ? cols[(int64_t)o + lane] : -1;
-   const int32_t c1 = w > 0 ? cols[(int64_t)o + (int64_t)(w - 1) / 2 * kSellSlice + lane] : -1;
-   const int valid = __syncthreads_count(c0 >= 0) + __syncthreads_count(c1 >= 0);
-   const int inside = __syncthreads_count((uint32_t)(c0 - lo) < width) + __syncthreads_count((uint32_t)(c1 - lo) < width);
-   const bool staged = 2 * inside >= valid;
-   if (staged) {
-      for (uint32_t j = threadIdx.x; j < width; j += kWindowThreads) win[j] = x[lo + j];
-      __syncthreads();
-   }
-   const uint32_t reach = staged ? width : 0u;
+   for (uint32_t j = threadIdx.x; j < width; j += kWindowThreads) win[j] = x[lo + j];
+   __syncthreads();
    for (; s < s1; s += kWindowWarps) {
       const int32_t* C = cols + o + lane;
       const Real* V = vals + o + lane;
@@ -295,7 +320,7 @@ __global__ void __launch_bounds__(kWindowThreads, 1)
 #pragma unroll
          for (int u = 0; u < kWindowDepth; u++) {
             const uint32_t at = (uint32_t)(c[u] - lo);
-            if (at < reach)
+            if (at < width)
                part[u & 3] += v[u] * win[at];
             else if (c[u] >= 0)
                part[u & 3] += v[u] * ld_gather(x + c[u]);
@@ -306,33 +331,32 @@ __global__ void __launch_bounds__(kWindowThreads, 1)
    }
 }
 
-// Launches k_sell_window where it is expected to be the faster one (false:
-// not launched).
+// Launches k_sell_window where it is expected to be the faster one; *out the runs
+// that it may have taken (per_block 0: not launched).
 template <typename Real>
-bool launch_window(const tnlb_segments* seg, int32_t columns, const int32_t* cols, const Real* vals, const Real* x,
-                   Real* y, Real alpha, Real beta, int32_t begin, int32_t end, cudaStream_t st, cudaError_t* e)
+void launch_window(const tnlb_segments* seg, int32_t columns, const int32_t* cols, const Real* vals, const Real* x,
+                   Real* y, Real alpha, Real beta, int32_t begin, int32_t end, cudaStream_t st, SellWindow* out)
 {
    int dev = 0, sms = 0, smem = 0;
    if (cudaGetDevice(&dev) != cudaSuccess ||
        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
        cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) {
       cudaGetLastError();
-      return false;
+      return;
    }
    // at least two slices a warp, and a window of three times the block's rows
-   const int32_t per_block = (seg->slices + sms - 1) / sms;
+   const int32_t per_block = ((seg->slices + sms - 1) / sms + 7) / 8 * 8;
    const int32_t room = (int32_t)(smem / sizeof(Real));
-   if (per_block < 2 * kWindowWarps || (int64_t)per_block * kSellSlice * 3 > room) return false;
+   if (per_block < 2 * kWindowWarps || (int64_t)per_block * kSellSlice * 3 > room) return;
    auto* k = k_sell_window<Real>;
    if (cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
       cudaGetLastError();
-      return false;
+      return;
    }
    k<<<(seg->slices + per_block - 1) / per_block, kWindowThreads, (size_t)room * sizeof(Real), st>>>(
       cols, vals, x, y, seg->slice_offsets.as<int32_t>(), seg->slice_segment_sizes.as<int32_t>(), seg->slices,
-      per_block, columns, room, begin, end, alpha, beta);
-   *e = cudaGetLastError();
-   return true;
+      SellWindow{per_block, columns, room}, begin, end, alpha, beta);
+   *out = SellWindow{per_block, columns, room};
 }
 
 template <typename Real, int G>
@@ -614,11 +638,11 @@ tnlb_status launch(const tnlb_segments* seg, const int32_t* cols, const Real* va
                G = mean_w >= 256 ? 8 : (mean_w >= 64 ? 4 : (mean_w >= 16 ? 2 : 1));
             }
             // narrow slices are stencils, whose lanes gather neighbours
-            cudaError_t e = cudaSuccess;
-            if (kernel == TNLB_KERNEL_DEFAULT && tps <= 0 && G >= 2 && G <= 4 &&
-                launch_window<Real>(seg, columns, cols, vals, x, y, alpha, beta, begin, end, st, &e)) {
-               TNLB_CUDA_TRY(e);
-               break;
+            SellWindow win{};
+            if (kernel == TNLB_KERNEL_DEFAULT && tps <= 0 && G >= 2 && G <= 4) {
+               launch_window<Real>(seg, columns, cols, vals, x, y, alpha, beta, begin, end, st, &win);
+               TNLB_CHECK_LAUNCH();
+               if (win.per_block > 0) *launches = 1;
             }
             const int32_t* so = seg->slice_offsets.as<int32_t>();
             const int32_t* sw = seg->slice_segment_sizes.as<int32_t>();
@@ -633,11 +657,11 @@ tnlb_status launch(const tnlb_segments* seg, const int32_t* cols, const Real* va
                      k<<<g, 256, 0, st>>>(cols, vals, x, y, so, sw, seg->slices, begin, end, alpha, beta);
                   }
                   else
-                     k_sell_col<Real, 1><<<grid_for(seg->slices, 8), 256, 0, st>>>(cols, vals, x, y, so, sw, seg->slices, begin, end, alpha, beta);
+                     k_sell_col<Real, 1><<<grid_for(seg->slices, 8), 256, 0, st>>>(cols, vals, x, y, so, sw, seg->slices, begin, end, alpha, beta, win);
                   break;
-               case 2: k_sell_col<Real, 2><<<grid_for(seg->slices, 4), 256, 0, st>>>(cols, vals, x, y, so, sw, seg->slices, begin, end, alpha, beta); break;
-               case 4: k_sell_col<Real, 4><<<grid_for(seg->slices, 2), 256, 0, st>>>(cols, vals, x, y, so, sw, seg->slices, begin, end, alpha, beta); break;
-               case 8: k_sell_col<Real, 8><<<grid_for(seg->slices, 1), 256, 0, st>>>(cols, vals, x, y, so, sw, seg->slices, begin, end, alpha, beta); break;
+               case 2: k_sell_col<Real, 2><<<grid_for(seg->slices, 4), 256, 0, st>>>(cols, vals, x, y, so, sw, seg->slices, begin, end, alpha, beta, win); break;
+               case 4: k_sell_col<Real, 4><<<grid_for(seg->slices, 2), 256, 0, st>>>(cols, vals, x, y, so, sw, seg->slices, begin, end, alpha, beta, win); break;
+               case 8: k_sell_col<Real, 8><<<grid_for(seg->slices, 1), 256, 0, st>>>(cols, vals, x, y, so, sw, seg->slices, begin, end, alpha, beta, win); break;
                default: set_error("threads per segment must be 1, 2, 4 or 8 for column-major SlicedEllpack"); return TNLB_ERR_INVALID_ARGUMENT;
             }
          }
@@ -687,7 +711,7 @@ tnlb_status launch(const tnlb_segments* seg, const int32_t* cols, const Real* va
       default: set_error("format has no Ellpack-family kernel"); return TNLB_ERR_INVALID_ARGUMENT;
    }
    TNLB_CHECK_LAUNCH();
-   *launches = 1;
+   *launches += 1;
    return TNLB_OK;
 }
 
