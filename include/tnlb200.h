@@ -578,6 +578,11 @@ tnlb_status tnlb_precond_solve(const tnlb_precond* precond, const void* d_b, voi
 tnlb_status tnlb_precond_read_factor(const tnlb_precond* precond, int32_t which, int32_t* h_rowptr, int32_t* h_cols,
                                      void* h_values, int64_t capacity);
 
+/* How an ILU preconditioner solves its triangles: parts[0] and parts[1] are
+ * the thread blocks of the pipelined solves with L and U, 0 when they are
+ * solved level by level. */
+tnlb_status tnlb_precond_ilu_parts(const tnlb_precond* precond, int32_t* parts);
+
 /* Release a preconditioner.  Accepts NULL. */
 tnlb_status tnlb_precond_destroy(tnlb_precond* precond);
 

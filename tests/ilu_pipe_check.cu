@@ -6,8 +6,11 @@
 // as the waits of its external entries allow, finishes (no deadlock) with
 // every entry reading the row it means: from the ring slot that holds it, or
 // from a row its owner has finished -- for the part's own old rows so long
-// ago that the stage's refill cannot overtake it.  Prints one line
-// "ok <entries>" or the first violation.
+// ago that the stage's refill cannot overtake it.  And the choice of parts: a
+// chain of rows up to 8M long, one or eight entries a row, is one part, as
+// long as its steps one after the other, whatever parts it is cut into; grids
+// keep their parts and are a fraction of their one-part length.  Prints one
+// line "ok <entries>" or the first violation.
 #include <cstdint>
 #include <cstdio>
 #include <random>
@@ -125,10 +128,57 @@ void grid(int nx, int ny, int nz, bool upper, std::vector<int32_t>& rp, std::vec
          }
 }
 
+// every row depends on the `width` rows before it (upper: after it)
+int check_chain(int32_t n, int32_t width, bool upper)
+{
+   std::vector<int32_t> beg(n), end(n), cols;
+   cols.reserve((size_t)n * width);
+   for (int32_t i = 0; i < n; i++) {
+      beg[i] = (int32_t)cols.size();
+      for (int32_t d = 1; d <= width; d++) {
+         const int32_t c = upper ? i + d : i - d;
+         if (c >= 0 && c < n) cols.push_back(c);
+      }
+      end[i] = (int32_t)cols.size();
+   }
+   std::vector<int32_t> lev(n), level(n + 1);
+   for (int32_t i = 0; i < n; i++) lev[i] = upper ? n - 1 - i : i;
+   for (int32_t i = 0; i <= n; i++) level[i] = i;
+   const int32_t parts = pipe_parts(n, 148);
+   double ns = 0;
+   const PipePlan P = pipe_choose(lev, level, parts, beg, end, 0, cols, upper, &ns);
+   if (P.parts != 1 || ns < kPipeStepNs * n) return fail("chain in several parts", n, P.parts, 0);
+   const PipePlan Q = pipe_plan(lev, n - 1, parts);
+   if (pipe_schedule_ns(Q, beg, end, 0, cols, upper) < kPipeStepNs * n) return fail("chain too short", n, parts, 0);
+   return 0;
+}
+
+int check_grid_choice(int nx, int ny)
+{
+   std::vector<int32_t> rp, cols;
+   grid(nx, ny, 1, false, rp, cols);
+   const int32_t n = nx * ny, parts = pipe_parts(n, 148);
+   std::vector<int32_t> lev(n), level(nx + ny, 0), beg(rp.begin(), rp.end() - 1), end(rp.begin() + 1, rp.end());
+   for (int32_t i = 0; i < n; i++) level[(lev[i] = i % nx + i / nx) + 1]++;
+   for (size_t l = 1; l < level.size(); l++) level[l] += level[l - 1];
+   double ns = 0;
+   const PipePlan P = pipe_choose(lev, level, parts, beg, end, 0, cols, false, &ns);
+   double one = 0;
+   for (size_t l = 0; l + 1 < level.size(); l++) one += kPipeStepNs * ((level[l + 1] - level[l] + 255) / 256);
+   if (P.parts != parts || ns < kPipeStepNs * (nx + ny - 1) || ns > 0.7 * (one + kPipeRowNs * n))
+      return fail("grid's choice", n, P.parts, 0);
+   return 0;
+}
+
 }  // namespace
 
 int main()
 {
+   for (bool upper : {false, true})
+      for (int32_t n : {20000, 1000003, 4000000, 8000000})
+         for (int32_t width : {1, 8})
+            if ((int64_t)n * width <= 16000000 && check_chain(n, width, upper)) return 1;
+   if (check_grid_choice(1000, 1024) || check_grid_choice(700, 1900)) return 1;
    std::mt19937 rng(1);
    std::vector<int32_t> rp, cols;
    const int sizes[][3] = {{1, 1, 1}, {5, 7, 1}, {300, 1, 1}, {257, 255, 1}, {1, 600, 1}, {31, 33, 29}, {700, 90, 1}};

@@ -141,6 +141,7 @@ tnlb_precond_create_fsai = _sig("tnlb_precond_create_fsai", [_p, C.c_int, _p, _p
 tnlb_precond_create = _sig("tnlb_precond_create", [C.c_int, _p, C.c_int, _p, _p, _p, C.POINTER(_p)])
 tnlb_precond_solve = _sig("tnlb_precond_solve", [_p, _p, _p, _p])
 tnlb_precond_destroy = _sig("tnlb_precond_destroy", [_p])
+tnlb_precond_ilu_parts = _sig("tnlb_precond_ilu_parts", [_p, _p])
 tnlb_precond_read_factor = _sig("tnlb_precond_read_factor", [_p, _i32, _p, _p, _p, _i64])
 tnlb_solve_preconditioned = _sig("tnlb_solve_preconditioned", [C.c_int, _p, C.POINTER(SolverParams), _p, C.c_int, _p,
                                                                _p, _p, _p, _p, C.POINTER(SolveResult)])

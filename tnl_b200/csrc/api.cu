@@ -506,6 +506,15 @@ tnlb_status tnlb_precond_read_factor(const tnlb_precond* precond, int32_t which,
    return TNLB_OK;
 }
 
+tnlb_status tnlb_precond_ilu_parts(const tnlb_precond* precond, int32_t* parts)
+{
+   clear_error();
+   TNLB_REQUIRE(precond && parts, TNLB_ERR_INVALID_ARGUMENT, "null argument");
+   TNLB_REQUIRE(precond->ilu, TNLB_ERR_INVALID_ARGUMENT, "not an ILU preconditioner");
+   tnlb::ilu0_parts(precond->ilu, parts);
+   return TNLB_OK;
+}
+
 tnlb_status tnlb_precond_destroy(tnlb_precond* precond)
 {
    clear_error();

@@ -165,19 +165,23 @@ __device__ __forceinline__ void band_copy(void* dst, const void* src, uint32_t b
                 : "memory");
 }
 
-// Polls the mbarrier's phase `parity` at most `tries` times.
-__device__ __forceinline__ bool band_wait(uint64_t* bar, uint32_t parity, long tries = kBandSpin)
+// One poll of the mbarrier's phase `parity`.
+__device__ __forceinline__ bool band_try(uint64_t* bar, uint32_t parity)
 {
-   const uint32_t a = band_smem(bar);
-   for (long it = 0; it < tries; it++) {
-      uint32_t done;
-      asm volatile(
-         "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-         : "=r"(done)
-         : "r"(a), "r"(parity)
-         : "memory");
-      if (done) return true;
-   }
+   uint32_t done;
+   asm volatile(
+      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(done)
+      : "r"(band_smem(bar)), "r"(parity)
+      : "memory");
+   return done != 0;
+}
+
+// Polls the mbarrier's phase `parity` at most kBandSpin times.
+__device__ __forceinline__ bool band_wait(uint64_t* bar, uint32_t parity)
+{
+   for (long it = 0; it < kBandSpin; it++)
+      if (band_try(bar, parity)) return true;
    return false;
 }
 

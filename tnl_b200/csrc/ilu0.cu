@@ -22,7 +22,6 @@
 
 #include "ilu_pipe.cuh"
 #include "internal.cuh"
-#include "reduce.cuh"
 #include "segview.cuh"
 
 namespace tnlb {
@@ -291,26 +290,26 @@ struct PipeTri {
    // progress[parts * 32] is followed, at the same place for both
    // triangles, by the error word of the last (unused) part's slot.
    template <bool Upper>
-   tnlb_status launch(const Real* in, Real* out, const Real* ext_src, int32_t* pr, cudaStream_t st) const
+   tnlb_status launch(const Real* in, Real* out, const Real* ext_src, int32_t* pr, int32_t* failed,
+                      cudaStream_t st) const
    {
       PipeArgs<Real> a{steps.as<PipeStep>(), part_step.as<int32_t>(), packed.as<unsigned char>(), in,
-                       ext.as<PipeExt>(), ext_src, out, pr, pr + kPipeMaxParts * 32, lay, consumers};
+                       ext.as<PipeExt>(), ext_src, out, pr, pr + kPipeMaxParts * 32, failed, lay, consumers};
       void* args[] = {&a};
       TNLB_CUDA_TRY(cudaLaunchCooperativeKernel(kernel<Upper>(K), dim3(parts), dim3(32 * (consumers + 3 + lay.stages)),
                                                 args, smem(), st));
       return TNLB_OK;
    }
 
-   // The packed triangle of `plan`; beg/end delimit the entries of a row,
-   // `skip` of them not taken (U's pivot).  K stays 0 when a step has more
-   // external entries than a stage holds, or the plan is not worth it
-   // against `other_ns` of the level-by-level solve.
+   // The packed triangle of `plan`, whose schedule takes `own_ns`; beg/end
+   // delimit the entries of a row, `skip` of them not taken (U's pivot).  K
+   // stays 0 when a step has more external entries than a stage holds, or the
+   // plan is not worth it against `other_ns` of the level-by-level solve.
    template <bool Upper>
    tnlb_status build(PipePlan& plan, const PipeBuild& dev, int32_t k, const Real* lu, const int32_t* dst_of,
-                     double other_ns, cudaStream_t st)
+                     double own_ns, double other_ns, cudaStream_t st)
    {
       const int32_t ns = (int32_t)plan.steps.size();
-      const int64_t n = (int64_t)plan.pos.size();
       DeviceBuffer count;
       TNLB_TRY_STATUS(count.alloc(sizeof(int32_t) * (size_t)ns));
       TNLB_CUDA_TRY(cudaMemsetAsync(count.ptr, 0, sizeof(int32_t) * (size_t)ns, st));
@@ -327,10 +326,10 @@ struct PipeTri {
          plan.steps[s].ext1 = (int32_t)total;
          emax = std::max(emax, ec[s]);
       }
-      // a step about 230 ns, a row 0.5, an external entry 3, a part's lag 2200
-      const double ns_est =
-         230.0 * plan.max_steps + (0.5 * (double)n + 3.0 * (double)total) / plan.parts + 2200.0 * plan.parts;
-      if (ns_est >= other_ns || plan.max_steps >= kPipeMaxNeed) return TNLB_OK;
+      // an external entry about 3 ns
+      if (own_ns + 3.0 * (double)total / plan.parts >= other_ns ||
+          (plan.parts > 1 && plan.max_steps >= kPipeMaxNeed))
+         return TNLB_OK;
       const int32_t kk = k <= 4 ? std::max(k, 1) : 8;
       const int32_t row_bytes = row_size<Upper>(kk);
       consumers = (plan.max_rows + 31) / 32;
@@ -343,7 +342,7 @@ struct PipeTri {
       lay.stages = (int32_t)std::min<int64_t>(fit, kPipeMaxStages);
       lay.stage_bytes = (int32_t)bytes;
       parts = plan.parts;
-      npad = plan.npad;
+      npad = (int32_t)plan.npad;
       TNLB_TRY_STATUS(packed.alloc((size_t)npad * row_bytes));
       TNLB_TRY_STATUS(ext.alloc(sizeof(PipeExt) * (size_t)total));
       TNLB_CUDA_TRY(cudaMemcpyAsync(steps.ptr, plan.steps.data(), sizeof(PipeStep) * (size_t)ns,
@@ -387,6 +386,9 @@ struct PipeTri {
 struct Ilu0Base {
    virtual ~Ilu0Base() = default;
    virtual tnlb_status apply(const void* b, void* x, cudaStream_t st) = 0;
+   // Whether the applications that have finished on the device did so properly.
+   virtual tnlb_status check() = 0;
+   virtual void parts(int32_t* of) const = 0;  // of L's and U's pipelines
 };
 
 template <typename Real>
@@ -397,8 +399,10 @@ struct Ilu0 : Ilu0Base {
    // off-diagonal U entries): strides kl / ku
    int kl = 0, ku = 0;
    DeviceBuffer lpc, lpv, upc, upv, udv, perm;
-   PipeTri<Real> lpipe, upipe;  // the pipelined form of both solves (ilu_pipe.cuh), where it is taken
+   bool pipe = false;  // whether the solves run as pipelines (ilu_pipe.cuh)
+   PipeTri<Real> lpipe, upipe;
    DeviceBuffer lin, uin, progress;
+   int32_t* pipe_failed = nullptr;  // host memory that the pipeline's kernels write when a wait runs out
    std::vector<int32_t> lptr, uptr;  // level boundaries into lrows / urows
    cudaGraphExec_t exec = nullptr;
    const Real* g_b = nullptr;
@@ -409,6 +413,7 @@ struct Ilu0 : Ilu0Base {
    {
       if (exec) cudaGraphExecDestroy(exec);
       if (cs) cudaStreamDestroy(cs);
+      if (pipe_failed) cudaFreeHost(pipe_failed);
    }
 
    template <int KL, int KU>
@@ -519,15 +524,29 @@ struct Ilu0 : Ilu0Base {
       k_pipe_start<Real><<<grid_for(std::max(lpipe.npad, 2 * flags), 256), 256, 0, st>>>(
          lpipe.rows_at.template as<int32_t>(), lpipe.npad, b, lin.as<Real>(), pr, 2 * flags);
       TNLB_CHECK_LAUNCH();
-      TNLB_TRY_STATUS((lpipe.template launch<false>(lin.as<Real>(), uin.as<Real>(), uin.as<Real>(), pr, st)));
-      return upipe.template launch<true>(uin.as<Real>(), x, x, pr + flags, st);
+      TNLB_TRY_STATUS((lpipe.template launch<false>(lin.as<Real>(), uin.as<Real>(), uin.as<Real>(), pr, pipe_failed, st)));
+      return upipe.template launch<true>(uin.as<Real>(), x, x, pr + flags, pipe_failed, st);
+   }
+
+   void parts(int32_t* of) const override
+   {
+      of[0] = pipe ? lpipe.parts : 0;
+      of[1] = pipe ? upipe.parts : 0;
+   }
+
+   tnlb_status check() override
+   {
+      if (!pipe_failed || !*(volatile int32_t*)pipe_failed) return TNLB_OK;
+      *(volatile int32_t*)pipe_failed = 0;
+      set_error("ILU solve: a wait between blocks ran out");
+      return TNLB_ERR_CUDA;
    }
 
    tnlb_status apply(const void* bv, void* xv, cudaStream_t st) override
    {
       const Real* b = static_cast<const Real*>(bv);
       Real* x = static_cast<Real*>(xv);
-      if (lpipe.K > 0) return apply_pipe(b, x, st);
+      if (pipe) return apply_pipe(b, x, st);
       // Solves are replayed from a graph captured for fixed (b, x) buffers:
       // copy in/out of the graph's own buffers when the caller's differ.
       if (!exec) {
@@ -614,10 +633,13 @@ tnlb_status create_from_factors_t(int32_t n, const std::vector<int32_t>& rp, con
 // The pipelined form of both triangular solves where it is expected to be
 // faster than the level-by-level one, by times measured on 5- and 7-point
 // grids: a level of at most kIluPipeThreads rows 1.0 us, a larger one 2.3 us
-// plus its rows' 60 bytes at 3 TB/s.
+// plus its rows' 60 bytes at 3 TB/s.  Row i's entries: L [ls, us), U [us, ue)
+// with the pivot first.
 template <typename Real>
 tnlb_status build_pipe(Ilu0<Real>* P, const std::vector<int32_t>& llev, const std::vector<int32_t>& ulev,
-                       int32_t lmax, int32_t umax, int32_t ml, int32_t mu, cudaStream_t st)
+                       const std::vector<int32_t>& ls, const std::vector<int32_t>& us,
+                       const std::vector<int32_t>& ue, const std::vector<int32_t>& hcols, int32_t ml, int32_t mu,
+                       cudaStream_t st)
 {
    auto level_ns = [](const std::vector<int32_t>& ptr) {
       double t = 0;
@@ -631,34 +653,34 @@ tnlb_status build_pipe(Ilu0<Real>* P, const std::vector<int32_t>& llev, const st
    TNLB_CUDA_TRY(cudaGetDevice(&dev));
    TNLB_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
    const int32_t parts = pipe_parts(P->n, sms);
-   const double least = 2200.0 * parts + 0.5 * P->n / parts;  // with no level at all
+   const double least = kPipeLagNs * parts + kPipeRowNs * P->n / parts;  // with no level at all
    if (least >= level_ns(P->lptr) || least >= level_ns(P->uptr)) return TNLB_OK;
-   PipePlan L = pipe_plan(llev, lmax, parts), U = pipe_plan(ulev, umax, parts);
+   double l_ns = 0, u_ns = 0;
+   PipePlan L = pipe_choose(llev, P->lptr, parts, ls, us, 0, hcols, false, &l_ns);
+   PipePlan U = pipe_choose(ulev, P->uptr, parts, us, ue, 1, hcols, true, &u_ns);
+   if (L.npad > INT32_MAX || U.npad > INT32_MAX) return TNLB_OK;
    DeviceBuffer lpos, lstep, upos, ustep;
    TNLB_TRY_STATUS(P->lpipe.upload(L, lpos, lstep, st));
    TNLB_TRY_STATUS(P->upipe.upload(U, upos, ustep, st));
    const int32_t* cols = P->cols.template as<int32_t>();
    auto i32 = [](const DeviceBuffer& d) { return d.as<int32_t>(); };
    const PipeBuild bl{i32(P->lpipe.rows_at), i32(lpos), i32(lstep), i32(P->lstart), i32(P->ustart), cols,
-                      i32(P->lpipe.part_step), P->lpipe.steps.template as<PipeStep>(), L.npad, L.chunk, 0};
+                      i32(P->lpipe.part_step), P->lpipe.steps.template as<PipeStep>(), (int32_t)L.npad, L.chunk, 0};
    const PipeBuild bu{i32(P->upipe.rows_at), i32(upos), i32(ustep), i32(P->ustart), i32(P->uend), cols,
-                      i32(P->upipe.part_step), P->upipe.steps.template as<PipeStep>(), U.npad, U.chunk, 1};
+                      i32(P->upipe.part_step), P->upipe.steps.template as<PipeStep>(), (int32_t)U.npad, U.chunk, 1};
    const Real* lu = P->lu.template as<Real>();
-   TNLB_TRY_STATUS(P->upipe.template build<true>(U, bu, mu, lu, nullptr, level_ns(P->uptr), st));
-   if (P->upipe.K > 0)
-      TNLB_TRY_STATUS(P->lpipe.template build<false>(L, bl, ml, lu, i32(upos), level_ns(P->lptr), st));
-   if (P->lpipe.K == 0) {
-      for (PipeTri<Real>* t : {&P->lpipe, &P->upipe}) {
-         t->K = 0;
-         for (DeviceBuffer* d : {&t->steps, &t->part_step, &t->rows_at, &t->packed, &t->ext}) d->release();
-      }
-      return TNLB_OK;
-   }
+   TNLB_TRY_STATUS(P->upipe.template build<true>(U, bu, mu, lu, nullptr, u_ns, level_ns(P->uptr), st));
+   if (P->upipe.K == 0) return TNLB_OK;
+   TNLB_TRY_STATUS(P->lpipe.template build<false>(L, bl, ml, lu, i32(upos), l_ns, level_ns(P->lptr), st));
+   if (P->lpipe.K == 0) return TNLB_OK;
    TNLB_TRY_STATUS(P->lin.alloc(sizeof(Real) * (size_t)L.npad));
    TNLB_TRY_STATUS(P->uin.alloc(sizeof(Real) * (size_t)U.npad));
    TNLB_TRY_STATUS(P->progress.alloc(sizeof(int32_t) * 2 * (kPipeMaxParts + 1) * 32));
+   TNLB_CUDA_TRY(cudaHostAlloc((void**)&P->pipe_failed, sizeof(int32_t), cudaHostAllocMapped | cudaHostAllocPortable));
+   *P->pipe_failed = 0;
    TNLB_CUDA_TRY(cudaMemsetAsync(P->uin.ptr, 0, sizeof(Real) * (size_t)U.npad, st));  // the padding is copied, not used
    TNLB_CUDA_TRY(cudaStreamSynchronize(st));
+   P->pipe = true;
    return TNLB_OK;
 }
 
@@ -736,11 +758,23 @@ tnlb_status analyze_t(Ilu0<Real>* P, const std::vector<int32_t>& rp, const std::
       ml = std::max(ml, us[i] - ls[i]);
       mu = std::max(mu, ue[i] - us[i] - 1);
    }
-   if (ml <= 8 && mu <= 8 && ordered) TNLB_TRY_STATUS(build_pipe(P, llev, ulev, lmax, umax, ml, mu, st));
-   if (P->lpipe.K > 0) {
+   if (ml <= 8 && mu <= 8 && ordered) {
+      const tnlb_status s = build_pipe(P, llev, ulev, ls, us, ue, cols, ml, mu, st);
+      // its packed rows take up to four times a chain's: without room for them the levels do
+      if (s != TNLB_OK && s != TNLB_ERR_OUT_OF_MEMORY) return s;
+      if (s != TNLB_OK) {
+         cudaGetLastError();
+         clear_error();
+      }
+   }
+   if (P->pipe) {
       for (DeviceBuffer* d : {&P->lrows, &P->urows, &P->dlptr, &P->duptr}) d->release();
       return TNLB_OK;
    }
+   for (PipeTri<Real>* t : {&P->lpipe, &P->upipe})
+      for (DeviceBuffer* d : {&t->steps, &t->part_step, &t->rows_at, &t->packed, &t->ext}) d->release();
+   P->lin.release();
+   P->uin.release();
    if (ml <= 8 && mu <= 8) {
       auto stride = [](int32_t m) { return m <= 1 ? 1 : m <= 2 ? 2 : m <= 4 ? 4 : 8; };
       const int kl = stride(ml), ku = stride(mu);
@@ -829,6 +863,10 @@ tnlb_status ilu0_apply(void* ilu, const void* b, void* x, cudaStream_t st)
 {
    return static_cast<Ilu0Base*>(ilu)->apply(b, x, st);
 }
+
+tnlb_status ilu0_check(void* ilu) { return static_cast<Ilu0Base*>(ilu)->check(); }
+
+void ilu0_parts(void* ilu, int32_t* parts) { static_cast<Ilu0Base*>(ilu)->parts(parts); }
 
 void ilu0_destroy(void* ilu) { delete static_cast<Ilu0Base*>(ilu); }
 

@@ -5,8 +5,8 @@
 // in natural order has about 2N of them with at most N rows each, so what
 // counts is the time from one level to the next.  One block walking the
 // levels with x in global memory took 1.03 us a level, two solves of the
-// 1000 x 1024 grid's FP64 factors 4.2 ms; here a level takes 0.23 us and
-// they take 0.97 ms.
+// 1000 x 1024 grid's FP64 factors 4.2 ms; here a level takes 0.21 us and
+// they take 0.86 ms.
 //  * The rows are cut into P contiguous parts, one block each (all resident:
 //    cooperative launch).  A block walks its own rows level by level
 //    ("steps" of at most kPipeStepRows rows), one row per thread.
@@ -29,9 +29,12 @@
 // (separately rounded multiply and subtract, ascending columns, IEEE
 // division), so results keep their bits.
 //
-// Every wait is bounded.  A wait that runs out raises *err, and the values
-// it waited for become NaN; no wait of the launch lasts after that, and the
-// blocks run to their end.
+// Every wait is bounded: it runs out when no part has finished a step for
+// kPipePatience.  A part may lie behind a chain of others that solve one after
+// the other for seconds, so polls counted from the start of a wait say nothing.
+// A wait that runs out raises *err, which ends the others, and the host's
+// *failed, which the caller reports.  The block then takes no further step,
+// runs to its end and sets all its rows to NaN.
 #pragma once
 
 #include <algorithm>
@@ -105,7 +108,8 @@ struct PipeExt {
 // Host plan of one triangle: the steps of the parts, in order, and the
 // packed position of every row (each step starts at a multiple of 4).
 struct PipePlan {
-   int32_t parts = 1, chunk = 0, npad = 0, max_rows = 0, max_steps = 0;
+   int32_t parts = 1, chunk = 0, max_rows = 0, max_steps = 0;
+   int64_t npad = 0;
    std::vector<PipeStep> steps;
    std::vector<int32_t> part_step;  // [parts + 1]
    std::vector<int32_t> rows_at;    // [npad], -1 in the padding
@@ -117,7 +121,8 @@ struct PipePlan {
 // FP64, us an application: 100 x 100 (n = 10^4) P = 1 104, 4 116, 8 138;
 // 1000 x 1024 P = 1 2375, 4 1076, 8 939, 14 967, 20 997, 64 1275; 95 x 96 x
 // 97 P = 4 1062, 8 707, 14 557, 20 514, 32 590; 192^3 P = 14 3379, 32 2176,
-// 64 1946.
+// 64 1946.  (By waits counted from their start; the parts taken here now take
+// 105, 858 and 571.)
 inline int32_t pipe_parts(int64_t n, int32_t sms)
 {
    int32_t p = (int32_t)std::lround(std::sqrt((double)n / 5000.0));
@@ -165,10 +170,65 @@ inline PipePlan pipe_plan(const std::vector<int32_t>& lev, int32_t max_level, in
       P.part_step.push_back((int32_t)P.steps.size());
       P.max_steps = std::max(P.max_steps, P.part_step[p + 1] - P.part_step[p]);
    }
-   P.npad = (int32_t)t;
+   P.npad = t;
+   if (t > INT32_MAX) return P;  // positions past the index type: no plan
    P.rows_at.assign((size_t)P.npad, -1);
    for (int32_t i = 0; i < n; i++) P.rows_at[P.pos[i]] = i;
    return P;
+}
+
+// What a step takes at least, what each of its rows adds, and how long after a
+// step another part's step that needs it can start (ns, measured).
+constexpr double kPipeStepNs = 230.0, kPipeRowNs = 0.5, kPipeLagNs = 2200.0;
+
+// Length of the plan's schedule: a step follows the one before it in its part
+// and, by the lag, the steps of other parts that hold x of its entries
+// [beg[i] + skip, end[i]).  Parts that depend on one another's last rows
+// follow one another here as they do on the device.
+inline double pipe_schedule_ns(const PipePlan& P, const std::vector<int32_t>& beg, const std::vector<int32_t>& end,
+                               int32_t skip, const std::vector<int32_t>& cols, bool upper)
+{
+   const int64_t n = (int64_t)P.pos.size();
+   std::vector<double> done(P.steps.size(), 0.0);  // first the earliest start, then the end
+   double longest = 0.0;
+   for (int32_t q = 0; q < P.parts; q++) {
+      const int32_t p = upper ? P.parts - 1 - q : q;
+      const int32_t r0 = (int32_t)std::min<int64_t>(n, (int64_t)p * P.chunk);
+      const int32_t r1 = (int32_t)std::min<int64_t>(n, (int64_t)(p + 1) * P.chunk);
+      for (int32_t i = r0; i < r1; i++)
+         for (int32_t k = beg[i] + skip; k < end[i]; k++)
+            if (cols[k] < r0 || cols[k] >= r1)
+               done[P.step[i]] = std::max(done[P.step[i]], done[P.step[cols[k]]] + kPipeLagNs);
+      double t = 0.0;
+      for (int32_t s = P.part_step[p]; s < P.part_step[p + 1]; s++) {
+         t = std::max(t, done[s]) + kPipeStepNs + kPipeRowNs * P.steps[s].rows;
+         done[s] = t;
+      }
+      longest = std::max(longest, t);
+   }
+   return longest;
+}
+
+// The triangle's plan of `parts` parts and its length, or of one part where that
+// takes no longer: where the parts have to follow one another.  level: row counts'
+// prefix sums by level.
+inline PipePlan pipe_choose(const std::vector<int32_t>& lev, const std::vector<int32_t>& level, int32_t parts,
+                            const std::vector<int32_t>& beg, const std::vector<int32_t>& end, int32_t skip,
+                            const std::vector<int32_t>& cols, bool upper, double* ns)
+{
+   double one = 0.0;
+   for (size_t l = 0; l + 1 < level.size(); l++) {
+      const int32_t rows = level[l + 1] - level[l];
+      one += kPipeStepNs * ((rows + kPipeStepRows - 1) / kPipeStepRows) + kPipeRowNs * rows;
+   }
+   const int32_t max_level = (int32_t)level.size() - 2;
+   if (parts > 1) {
+      PipePlan P = pipe_plan(lev, max_level, parts);
+      *ns = pipe_schedule_ns(P, beg, end, skip, cols, upper);
+      if (*ns < one) return P;
+   }
+   *ns = one;
+   return pipe_plan(lev, max_level, 1);
 }
 
 // A packed row: K values, the pivot (upper), K codes, where the result goes
@@ -208,6 +268,8 @@ struct PipeLayout {
    int32_t stages, stage_bytes, in_off, ext_off;  // offsets within a stage
 };
 constexpr int32_t kPipeRows0 = 16;  // the packed rows' offset within a stage
+// Row count of every stage once the block takes no further step.
+constexpr int32_t kPipeNoRows = -1;
 
 template <typename Real>
 struct PipeArgs {
@@ -220,6 +282,7 @@ struct PipeArgs {
    Real* out;
    int32_t* progress;  // [parts * 32]: steps finished, one per 128 bytes
    int32_t* err;
+   int32_t* failed;  // host memory
    PipeLayout lay;
    int32_t consumers;  // warps
 };
@@ -247,17 +310,60 @@ __device__ __forceinline__ float pipe_ld_relaxed(const float* p)
    return v;
 }
 
+constexpr unsigned long long kPipePatience = 4000000000ull;  // ns
+constexpr int kPipeLook = 1024;                              // polls between two looks around
+
+// What a wait looks at while it lasts.
+struct PipePatience {
+   const int32_t* progress;
+   int32_t *err, *failed;
+   volatile int32_t* s_done;    // this block's steps finished
+   volatile int32_t* s_failed;  // this block has given up
+   uint32_t polls = 0, seen = 0;
+   unsigned long long since = 0;
+
+   // After a poll that found nothing: whether to go on.
+   __device__ __forceinline__ bool more()
+   {
+      if ((++polls & 63) != 0) return true;
+      return (polls & (kPipeLook - 1)) != 0 ? !*s_failed : look();
+   }
+   __device__ __forceinline__ bool look()
+   {
+      uint32_t now = (uint32_t)*s_done;
+#pragma unroll 1
+      for (int p = 0; p < (int)gridDim.x; p++) now += (uint32_t)pipe_ld_acquire(progress + p * 32);
+      unsigned long long t;
+      asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+      if (polls == kPipeLook || now != seen) {
+         seen = now;
+         since = t;
+      }
+      if (!*s_failed && !pipe_ld_acquire(err) && t - since < kPipePatience) return true;
+      *s_failed = 1;
+      atomicExch(err, 1);
+      asm volatile("st.relaxed.sys.global.s32 [%0], 1;" ::"l"(failed) : "memory");
+      return false;
+   }
+};
+
 // Waits until *flag >= need and returns *flag; -1 when the wait ran out here
 // or elsewhere.
-__device__ __forceinline__ int32_t pipe_wait(const int32_t* flag, int32_t need, int32_t* err)
+__device__ __forceinline__ int32_t pipe_wait(const int32_t* flag, int32_t need, PipePatience w)
 {
-   for (int it = 0; it < (1 << 22); it++) {
+   while (true) {
       const int32_t f = pipe_ld_acquire(flag);
       if (f >= need) return f;
-      if ((it & 1023) == 1023 && pipe_ld_acquire(err)) return -1;
+      if (!w.more()) return -1;
    }
-   atomicExch(err, 1);
-   return -1;
+}
+
+// Waits for the mbarrier's phase `parity`.
+__device__ __forceinline__ bool pipe_bar_wait(uint64_t* bar, uint32_t parity, PipePatience w)
+{
+   while (!band_try(bar, parity))
+      if (!w.more()) return false;
+   return true;
 }
 
 template <typename Real, int K, bool Upper>
@@ -267,14 +373,17 @@ __global__ void __launch_bounds__((kPipeMaxStages + 3) * 32 + kPipeStepRows, 1) 
    constexpr int32_t kB = (int32_t)sizeof(Real);
    extern __shared__ __align__(128) unsigned char smem[];
    __shared__ __align__(8) uint64_t s_full[kPipeMaxStages], s_empty[kPipeMaxStages];
-   __shared__ int32_t s_done;  // steps finished by the consumers
+   __shared__ int32_t s_done;     // steps finished by the consumers
+   __shared__ int32_t s_failed;   // a wait of this block ran out
    const int S = a.lay.stages, NC = a.consumers;
    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
    const int part = blockIdx.x;
    const int32_t first = a.part_step[part], count = a.part_step[part + 1] - first;
    if (threadIdx.x == 0) {
       s_done = 0;
+      s_failed = 0;
       for (int s = 0; s < S; s++) {
+         *reinterpret_cast<int32_t*>(smem + (size_t)kPipeWindow * kB + (size_t)s * a.lay.stage_bytes) = 0;
          asm volatile("mbarrier.init.shared::cta.b64 [%0], 2;" ::"r"(band_smem(&s_full[s])) : "memory");
          asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(band_smem(&s_empty[s])) : "memory");
       }
@@ -282,6 +391,10 @@ __global__ void __launch_bounds__((kPipeMaxStages + 3) * 32 + kPipeStepRows, 1) 
    }
    __syncthreads();
    if (count == 0) return;
+   const PipePatience patience{a.progress, a.err, a.failed, &s_done, &s_failed};
+   auto rows_of = [&](int s) {
+      return reinterpret_cast<int32_t*>(smem + (size_t)kPipeWindow * kB + (size_t)s * a.lay.stage_bytes);
+   };
    // the step barrier: consumers, the watcher and the keeper
    auto step_barrier = [&]() { asm volatile("bar.sync 1, %0;" ::"r"((NC + 2) * 32) : "memory"); };
 
@@ -340,11 +453,15 @@ __global__ void __launch_bounds__((kPipeMaxStages + 3) * 32 + kPipeStepRows, 1) 
       }
    }
    else if (warp == NC) {
-      // watcher: before step j starts, step j + 1 is there
+      // watcher: before step j starts, step j + 1 is there, or no stage has rows any more
       int s = 0;
       uint32_t parity = 0;
+      bool ok = true;
       auto arrived = [&]() {
-         if (!band_wait(&s_full[s], parity)) atomicExch(a.err, 1);
+         if (ok && !pipe_bar_wait(&s_full[s], parity, patience)) {
+            ok = false;
+            for (int q = 0; q < S; q++) atomicExch(rows_of(q), kPipeNoRows);
+         }
          if (++s == S) {
             s = 0;
             parity ^= 1u;
@@ -378,14 +495,17 @@ __global__ void __launch_bounds__((kPipeMaxStages + 3) * 32 + kPipeStepRows, 1) 
       // publisher: the steps finished, made visible to the other blocks
       if (lane == 0 && gridDim.x > 1) {
          int32_t seen = 0;
-         for (long it = 0; seen < count && it < kBandSpin; it++) {
+         PipePatience w = patience;
+         while (seen < count) {
             int32_t d;
             asm volatile("ld.acquire.cta.shared.s32 %0, [%1];" : "=r"(d) : "r"(band_smem(&s_done)) : "memory");
             if (d > seen) {
+               if (*const_cast<volatile int32_t*>(&s_failed)) break;  // steps after that hold no values
                pipe_st_release(a.progress + part * 32, d);
                seen = d;
-               it = 0;
             }
+            else if (!w.more())
+               break;
          }
       }
    }
@@ -398,7 +518,8 @@ __global__ void __launch_bounds__((kPipeMaxStages + 3) * 32 + kPipeStepRows, 1) 
       unsigned char* st = smem + (size_t)kPipeWindow * kB + (size_t)s * a.lay.stage_bytes;
       Real* ext = reinterpret_cast<Real*>(st + a.lay.ext_off);
       int32_t known_part = -1, known = 0;  // progress last read, and whose
-      uint32_t parity = 1;
+      uint32_t parity = 1, filled = 1;
+      int32_t rows = 0;  // as the stage's count says
       for (int32_t j = s; j < count; j += S) {
          const PipeStep d = a.steps[first + j];
          PipeExt e[E];
@@ -410,11 +531,16 @@ __global__ void __launch_bounds__((kPipeMaxStages + 3) * 32 + kPipeStepRows, 1) 
             }
          };
          entries(d.ext0);
+         bool more = true;
          if (lane == 0) {
-            if (j >= S && !band_wait(&s_empty[s], parity)) atomicExch(a.err, 1);
+            more = j < S || pipe_bar_wait(&s_empty[s], parity, patience);
+            more = more && atomicCAS(rows_of(s), rows, d.rows) == rows;
+         }
+         if (!__shfl_sync(0xffffffffu, (int)more, 0)) break;
+         rows = d.rows;
+         if (lane == 0) {
             const int rp = (d.rows + 3) & ~3;
             const uint32_t nb = (uint32_t)(rp * Row::kBytes), ni = (uint32_t)(rp * kB);
-            *reinterpret_cast<int32_t*>(st) = d.rows;
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             band_expect(&s_full[s], nb + ni);
             band_copy(st + kPipeRows0, a.packed + (size_t)d.t0 * Row::kBytes, nb, &s_full[s]);
@@ -431,7 +557,7 @@ __global__ void __launch_bounds__((kPipeMaxStages + 3) * 32 + kPipeStepRows, 1) 
                const int32_t need = (int32_t)(e[q].need & 0xffffffu), owner = (int32_t)(e[q].need >> 24);
                if (need > 0 && !(owner == known_part && known >= need)) {
                   known_part = owner;
-                  known = pipe_wait(a.progress + owner * 32, need, a.err);
+                  known = pipe_wait(a.progress + owner * 32, need, patience);
                }
                v[q] = need == 0 || known >= need ? pipe_ld_relaxed(a.ext_src + e[q].idx) : (Real)NAN;
             }
@@ -444,8 +570,18 @@ __global__ void __launch_bounds__((kPipeMaxStages + 3) * 32 + kPipeStepRows, 1) 
          __syncwarp();
          if (lane == 0) band_arrive(&s_full[s]);
          __syncwarp();
+         filled ^= 1u;
       }
+      // the last copies have landed before the block ends, also where nobody waited for them
+      if (lane == 0 && s < count) pipe_bar_wait(&s_full[s], filled, patience);
    }
+   __syncthreads();
+   if (*const_cast<volatile int32_t*>(&s_failed))
+      for (int32_t j = 0; j < count; j++) {
+         const PipeStep d = a.steps[first + j];
+         for (int32_t c = threadIdx.x; c < d.rows; c += blockDim.x)
+            a.out[reinterpret_cast<const int32_t*>(a.packed + (size_t)(d.t0 + c) * Row::kBytes)[Row::kInts + K]] = (Real)NAN;
+      }
 }
 
 // ----------------------------------------------------------------- set-up

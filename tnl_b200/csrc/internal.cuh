@@ -416,6 +416,8 @@ tnlb_status solve_mixed_reliable(const tnlb_segments* seg, const int32_t* cols, 
 tnlb_status ilu0_create(const tnlb_segments* seg, tnlb_real real, const int32_t* cols, const void* vals,
                         cudaStream_t st, void** out);
 tnlb_status ilu0_apply(void* ilu, const void* b, void* x, cudaStream_t st);
+// After a stream synchronisation: whether the applications before it succeeded.
+tnlb_status ilu0_check(void* ilu);
 // An ILU object over factors computed elsewhere (ILUT): host CSR whose row i
 // holds its L entries (columns < i) then its U entries (first = pivot).
 tnlb_status ilu_from_factors(tnlb_real real, int32_t n, const std::vector<int32_t>& rp,
@@ -423,6 +425,7 @@ tnlb_status ilu_from_factors(tnlb_real real, int32_t n, const std::vector<int32_
 tnlb_status ilut_create(const tnlb_segments* seg, tnlb_real real, const int32_t* cols, const void* vals, int32_t p,
                         double tau, cudaStream_t st, void** out);
 tnlb_status ilu0_read(void* ilu, int32_t* h_rowptr, int32_t* h_cols, void* h_vals, int64_t capacity, int real_bytes);
+void ilu0_parts(void* ilu, int32_t* parts);
 void ilu0_destroy(void* ilu);
 tnlb_status fsai_create(const tnlb_segments* seg, tnlb_real real, const int32_t* cols, const void* vals,
                         bool classical, cudaStream_t st, Fsai** out, bool two_factor = false, int level = 0);

@@ -2088,9 +2088,9 @@ tnlb_status idrs_solve(const Ctx<Real>& c, const Precond<Real>& Pc, const tnlb_s
 }
 
 template <typename Real>
-tnlb_status solve_t(tnlb_solver_kind solver, const tnlb_precond* pobj, const tnlb_solver_params& prm,
-                    const tnlb_segments* seg, tnlb_real real, const int32_t* cols, const Real* vals, const Real* b,
-                    Real* x, cudaStream_t st, tnlb_solve_result* res)
+tnlb_status run_solver(tnlb_solver_kind solver, const tnlb_precond* pobj, const tnlb_solver_params& prm,
+                       const tnlb_segments* seg, tnlb_real real, const int32_t* cols, const Real* vals, const Real* b,
+                       Real* x, cudaStream_t st, tnlb_solve_result* res)
 {
    Ctx<Real> c{seg, real, cols, vals, seg->n, st};
    const Precond<Real> P = view<Real>(pobj);
@@ -2107,6 +2107,15 @@ tnlb_status solve_t(tnlb_solver_kind solver, const tnlb_precond* pobj, const tnl
    }
    set_error("unknown solver");
    return TNLB_ERR_INVALID_ARGUMENT;
+}
+
+template <typename Real>
+tnlb_status solve_t(tnlb_solver_kind solver, const tnlb_precond* pobj, const tnlb_solver_params& prm,
+                    const tnlb_segments* seg, tnlb_real real, const int32_t* cols, const Real* vals, const Real* b,
+                    Real* x, cudaStream_t st, tnlb_solve_result* res)
+{
+   TNLB_TRY_STATUS(run_solver<Real>(solver, pobj, prm, seg, real, cols, vals, b, x, st, res));
+   return pobj && pobj->ilu ? ilu0_check(pobj->ilu) : TNLB_OK;
 }
 
 template <typename Real>
@@ -2224,7 +2233,7 @@ tnlb_status precond_apply(const tnlb_precond* P, const void* b, void* x, cudaStr
    else
       TNLB_TRY_STATUS(view<float>(P).apply(P->n, (const float*)b, (float*)x, st));
    TNLB_CUDA_TRY(cudaStreamSynchronize(st));
-   return TNLB_OK;
+   return P->ilu ? ilu0_check(P->ilu) : TNLB_OK;
 }
 
 // FP32 inner Krylov solve inside FP64 iterative refinement.
