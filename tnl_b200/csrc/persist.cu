@@ -1,7 +1,7 @@
 // persist.cu -- CG and BiCGStab iterations in one resident kernel.
 //
-// An iteration of CG on a matrix that fits L2 is three short passes over a few
-// vectors between two dot products; as separate launches each pass pays for
+// An iteration of CG on a matrix that fits L2 (persist_pays) is three short passes
+// over a few vectors between two dot products; as separate launches each pass pays for
 // its launch, its ramp and its tail, and every vector goes through memory.
 // Here one block per SM (cooperative launch, all resident) owns a contiguous
 // run of rows for the whole solve:
@@ -18,8 +18,6 @@
 //  * every block forms the scalars from the same totals, so all take the same
 //    branch.  Waits are bounded.
 // The row arithmetic and its order are those of the product kernels.
-#include <cooperative_groups.h>
-
 #include <cfloat>
 
 #include "persist.cuh"
@@ -743,6 +741,15 @@ bool persist_shape(const void* kernel, bool cluster, int64_t n, int vectors, int
    return true;
 }
 
+int64_t l2_bytes()
+{
+   int dev = 0, bytes = 0;
+   if (cudaGetDevice(&dev) != cudaSuccess ||
+       cudaDeviceGetAttribute(&bytes, cudaDevAttrL2CacheSize, dev) != cudaSuccess)
+      cudaGetLastError();
+   return bytes;
+}
+
 // `pick(sync)`: the kernel for PersistGrid or PersistCluster.
 template <typename Pick>
 PersistShape persist_choose(Pick&& pick, int64_t n, int vectors, int gathered, size_t real, int warp_stage)
@@ -773,7 +780,7 @@ int persist_stage(const tnlb_segments* seg)
 template <typename Real>
 PersistShape persist_cg(const tnlb_segments* seg)
 {
-   if (!persist_rows_fit(seg)) return {};
+   if (!persist_pays(seg, sizeof(Real), false, l2_bytes())) return {};
    return persist_choose([&](auto sync) { return TNLB_PERSIST_FORMAT(k_cg_persist, Real, decltype(sync), seg); },
                          seg->n, 4, 1, sizeof(Real), persist_stage<Real>(seg));
 }
@@ -781,7 +788,7 @@ PersistShape persist_cg(const tnlb_segments* seg)
 template <typename Real>
 PersistShape persist_bicgstab(const tnlb_segments* seg)
 {
-   if (!persist_rows_fit(seg)) return {};
+   if (!persist_pays(seg, sizeof(Real), true, l2_bytes())) return {};
    return persist_choose([&](auto sync) { return TNLB_PERSIST_FORMAT(k_bicg_persist, Real, decltype(sync), seg); },
                          seg->n, 6, 2, sizeof(Real), persist_stage<Real>(seg));
 }

@@ -8,7 +8,8 @@
 // dot product and norm is reduced on the device into a DevState record, and
 // the scalar recurrences (alpha, beta, residue, the stopping test) run in the
 // last block of the reduction.  CG and BiCGStab on short rows, with Jacobi or no
-// preconditioner, run in one resident kernel (persist.cu).  Otherwise CG's
+// preconditioner, run in one resident kernel (persist.cu) up to the sizes where it
+// is the faster one.  Otherwise CG's
 // iterations are captured in batches in a CUDA graph and replayed; kernels of
 // iterations past the stopping point return at once on the device `done` flag, so
 // the iteration count is exact; BiCGStab reads the state every iteration, and
