@@ -2,8 +2,9 @@
 FP64.
 
 Matrices at the rules' edges: columns inside the window, half outside, all
-over the place (the window is not taken), fewer and more columns than rows,
-and a last block and slice that are not full.  Bounds per row: 1e-13 (FP64)
+over the place (the window is not taken), some runs of rows one way and some
+the other, fewer and more columns than rows, and a last block and slice that
+are not full.  Bounds per row: 1e-13 (FP64)
 and 2e-5 (FP32) times the sum of the magnitudes that enter it, the repository's
 rule for a reordered sum.
 """
@@ -18,6 +19,7 @@ pytestmark = pytest.mark.gpu
 SHAPES = {  # rows, columns, half band (None: anywhere)
     "narrow": (310007, 310007, 400), "wide": (310007, 310007, 20000), "anywhere": (310007, 310007, None),
     "few_columns": (310007, 200003, 5000), "many_columns": (310007, 400009, 5000),
+    "mixed": (310007, 310007, "mixed"),  # first half of the rows in a band, the others anywhere
 }
 
 
@@ -30,6 +32,9 @@ def _matrix(rows, columns, half, longest, seed, triangle=False):
     row = np.repeat(np.arange(rows), lens)
     if half is None:
         cols = rng.integers(0, columns, len(row))
+    elif half == "mixed":
+        cols = np.where(row < rows // 2, np.clip(row + rng.integers(-400, 401, len(row)), 0, columns - 1),
+                        rng.integers(0, columns, len(row)))
     else:
         cols = np.clip(row + rng.integers(-half, half + 1, len(row)), 0, columns - 1)
     if triangle:
@@ -96,3 +101,22 @@ def test_symmetric_product(fmt, half, longest, real):
         want = want + 1.5 * np.bincount(r, v * x[c], minlength=n)
         scale = scale + 1.5 * np.bincount(r, np.abs(v * x[c]), minlength=n)
     _close(out, want, scale, real)
+
+
+@pytest.mark.parametrize("shape", ["narrow", "mixed", "anywhere"])
+def test_window_product_in_a_graph(shape):
+    """Captured, where the two kernels of a product follow one another, and replayed."""
+    import tnl_b200 as t
+
+    rows, columns, half = SHAPES[shape]
+    rp, cols, vals, _ = _matrix(rows, columns, half, 40, 3)
+    M = t.SparseMatrix(t.SlicedEllpack, torch.float64).assign(rp, cols, vals, columns)
+    x, y0 = (torch.tensor(v, device="cuda") for v in _vectors("float64", columns, rows))
+    want, out = y0.clone(), y0.clone()
+    M.vectorProduct(x, want, -1.5, 0.5)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        M.vectorProduct(x, out, -1.5, 0.5, synchronize=False)
+    out.copy_(y0)
+    graph.replay()
+    assert torch.equal(out, want)

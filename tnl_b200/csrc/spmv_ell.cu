@@ -102,8 +102,9 @@ __global__ void k_ell_row(const int32_t* __restrict__ cols, const Real* __restri
 
 // ------------------------------------------------------- SlicedEllpack
 
-// The runs of slices that k_sell_window takes, and the window of each: `room`
+// The runs of slices that k_sell_window may take, and the window of each: `room`
 // entries of x around the run's rows.
+constexpr int kWindowPercent = 60;
 struct SellWindow {
    int32_t per_block, columns, room;  // slices of a run, a multiple of 8; 0: no windows
    __device__ __forceinline__ int32_t lo(int64_t s0, int64_t s1) const
@@ -112,8 +113,8 @@ struct SellWindow {
       return (int32_t)imin64(imax64(mid - room / 2, 0), imax64((int64_t)columns - room, 0));
    }
    __device__ __forceinline__ uint32_t width(int32_t lo) const { return (uint32_t)imin64(room, columns - lo); }
-   // Whether most columns of run `b` lie in its window, from 32 slots of 8 of its
-   // slices.  Called by whole blocks of at least 256 threads; the answer is the
+   // Whether kWindowPercent of the columns of run `b` lie in its window, from 32
+   // slots of 8 of its slices.  Called by whole blocks of at least 256 threads; the answer is the
    // same in each.
    __device__ __forceinline__ bool taken(int32_t b, const int32_t* cols, const int32_t* slice_off,
                                          const int32_t* slice_w, int32_t slices) const
@@ -127,7 +128,7 @@ struct SellWindow {
          if (w > 0) c = cols[(int64_t)slice_off[s] + (int64_t)(w - 1) / 2 * kSellSlice + (threadIdx.x & 31)];
       }
       const int valid = __syncthreads_count(c >= 0);
-      return 2 * __syncthreads_count(c >= 0 && (uint32_t)(c - l) < width(l)) >= valid;
+      return 100 * __syncthreads_count(c >= 0 && (uint32_t)(c - l) < width(l)) >= kWindowPercent * valid;
    }
 };
 
@@ -141,9 +142,13 @@ __global__ void __launch_bounds__(256) k_sell_col(const int32_t* __restrict__ co
                                                   int32_t end, Real alpha, Real beta, SellWindow win)
 {
    __shared__ Real part[8][32];
-   if (win.per_block > 0 &&
-       win.taken((int32_t)((int64_t)blockIdx.x * (8 / G) / win.per_block), cols, slice_off, slice_w, slices))
-      return;
+   if (win.per_block > 0) {
+      const bool taken =
+         win.taken((int32_t)((int64_t)blockIdx.x * (8 / G) / win.per_block), cols, slice_off, slice_w, slices);
+      // this kernel may run beside k_sell_window, whose rows are others, but ends after it
+      if (blockIdx.x == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
+      if (taken) return;
+   }
    const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
    const int sub = wib % G;
    const int64_t slice = (int64_t)blockIdx.x * (8 / G) + wib / G;
@@ -266,13 +271,24 @@ __global__ void __launch_bounds__(256) k_sell_walk(const int32_t* __restrict__ c
 // slices keeps the x of its rows and of the columns around them in shared
 // memory.  Columns that differ from lane to lane take the L1 cache one lookup a
 // lane (27M of them, 96 us at one a cycle and SM), shared memory about 3.5
-// cycles for 32.  Nothing is known of the columns beforehand, so a block first
-// looks at some of its slots and leaves its run to k_sell_col, launched after it,
-// where most lie outside: gathers from memory want the L1 that the window takes,
-// 143 against 73 us for random columns at 500,000 rows (FP64).
-// FP32 residual at 1,000,003 rows of 9 to 45 entries in a band of 20,000: 102.6
-// us by two warps a slice, 82.4 so; its 370 MB with the padding take 57.
+// cycles for 32.  FP32 residual at 1,000,003 rows of 9 to 45 entries in a band of
+// 20,000: 102.9 us by two warps a slice, 81.9 so; its 370 MB with the padding take
+// 57.
+// Nothing is known of the columns beforehand, so a block first looks at some of
+// its slots and leaves its run to k_sell_col, launched behind it, where too many
+// lie outside: they want the L1 that the window takes, and 60% inside is where
+// both take the same (FP64, 27 entries a row in a band of 20,000 at 2,000,003 rows,
+// 62% inside: 201 us by a window, 229 by k_sell_col; in a band of 40,000 at 500,009
+// rows, 48% inside: 78 and 72).  163 KB leave enough L1 for the columns outside:
+// with 227 KB the same matrices took 209 and 88.
+// k_sell_col's blocks look at their run too, a wave of them 1.8 us.  So the window's
+// blocks let it start when they have their window, under their main loop (85.6 us
+// for the residual after 93.9); and those that leave their run end at once, so that
+// it finds the SMs empty and their L1 whole: random columns, 27 a row (FP64), at
+// 500,009 and 1,000,003 rows 73.8 and 129.1 us by k_sell_col alone, 76.8 and 134.2
+// behind the window's look; 138 and 169 when it starts earlier.
 constexpr int kWindowThreads = 1024, kWindowWarps = kWindowThreads / 32, kWindowDepth = 8;
+constexpr int kWindowBytes = 163 * 1024;
 extern __shared__ __align__(16) unsigned char window_smem[];
 
 template <typename Real>
@@ -296,6 +312,7 @@ __global__ void __launch_bounds__(kWindowThreads, 1)
    }
    for (uint32_t j = threadIdx.x; j < width; j += kWindowThreads) win[j] = x[lo + j];
    __syncthreads();
+   asm volatile("griddepcontrol.launch_dependents;");
    for (; s < s1; s += kWindowWarps) {
       const int32_t* C = cols + o + lane;
       const Real* V = vals + o + lane;
@@ -331,25 +348,50 @@ __global__ void __launch_bounds__(kWindowThreads, 1)
    }
 }
 
+// k_sell_col.  Behind k_sell_window (win) it starts once that kernel's blocks have
+// all looked at their runs, unless the stream is being captured.
+template <typename Real, int G>
+cudaError_t launch_sell_col(const tnlb_segments* seg, const int32_t* cols, const Real* vals, const Real* x, Real* y,
+                            Real alpha, Real beta, int32_t begin, int32_t end, const SellWindow& win, cudaStream_t st)
+{
+   cudaLaunchConfig_t cfg{};
+   cfg.gridDim = dim3(grid_for(seg->slices, 8 / G));
+   cfg.blockDim = dim3(256);
+   cfg.stream = st;
+   cudaLaunchAttribute at{};
+   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+   at.val.programmaticStreamSerializationAllowed = 1;
+   cfg.attrs = &at;
+   if (win.per_block > 0) {
+      cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+      const cudaError_t e = cudaStreamIsCapturing(st, &capture);
+      if (e != cudaSuccess) return e;
+      cfg.numAttrs = capture == cudaStreamCaptureStatusNone ? 1 : 0;
+   }
+   return cudaLaunchKernelEx(&cfg, k_sell_col<Real, G>, cols, vals, x, y,
+                             (const int32_t*)seg->slice_offsets.as<int32_t>(),
+                             (const int32_t*)seg->slice_segment_sizes.as<int32_t>(), seg->slices, begin, end, alpha,
+                             beta, win);
+}
+
 // Launches k_sell_window where it is expected to be the faster one; *out the runs
 // that it may have taken (per_block 0: not launched).
 template <typename Real>
 void launch_window(const tnlb_segments* seg, int32_t columns, const int32_t* cols, const Real* vals, const Real* x,
                    Real* y, Real alpha, Real beta, int32_t begin, int32_t end, cudaStream_t st, SellWindow* out)
 {
-   int dev = 0, sms = 0, smem = 0;
+   int dev = 0, sms = 0;
    if (cudaGetDevice(&dev) != cudaSuccess ||
-       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-       cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) {
+       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
       cudaGetLastError();
       return;
    }
-   // at least two slices a warp, and a window of three times the block's rows
+   // at least two slices a warp, and a window of at least twice the block's rows
    const int32_t per_block = ((seg->slices + sms - 1) / sms + 7) / 8 * 8;
-   const int32_t room = (int32_t)(smem / sizeof(Real));
-   if (per_block < 2 * kWindowWarps || (int64_t)per_block * kSellSlice * 3 > room) return;
+   const int32_t room = (int32_t)(kWindowBytes / sizeof(Real));
+   if (per_block < 2 * kWindowWarps || (int64_t)per_block * kSellSlice * 2 > room) return;
    auto* k = k_sell_window<Real>;
-   if (cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
+   if (cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, kWindowBytes) != cudaSuccess) {
       cudaGetLastError();
       return;
    }
@@ -657,11 +699,11 @@ tnlb_status launch(const tnlb_segments* seg, const int32_t* cols, const Real* va
                      k<<<g, 256, 0, st>>>(cols, vals, x, y, so, sw, seg->slices, begin, end, alpha, beta);
                   }
                   else
-                     k_sell_col<Real, 1><<<grid_for(seg->slices, 8), 256, 0, st>>>(cols, vals, x, y, so, sw, seg->slices, begin, end, alpha, beta, win);
+                     TNLB_CUDA_TRY((launch_sell_col<Real, 1>(seg, cols, vals, x, y, alpha, beta, begin, end, win, st)));
                   break;
-               case 2: k_sell_col<Real, 2><<<grid_for(seg->slices, 4), 256, 0, st>>>(cols, vals, x, y, so, sw, seg->slices, begin, end, alpha, beta, win); break;
-               case 4: k_sell_col<Real, 4><<<grid_for(seg->slices, 2), 256, 0, st>>>(cols, vals, x, y, so, sw, seg->slices, begin, end, alpha, beta, win); break;
-               case 8: k_sell_col<Real, 8><<<grid_for(seg->slices, 1), 256, 0, st>>>(cols, vals, x, y, so, sw, seg->slices, begin, end, alpha, beta, win); break;
+               case 2: TNLB_CUDA_TRY((launch_sell_col<Real, 2>(seg, cols, vals, x, y, alpha, beta, begin, end, win, st))); break;
+               case 4: TNLB_CUDA_TRY((launch_sell_col<Real, 4>(seg, cols, vals, x, y, alpha, beta, begin, end, win, st))); break;
+               case 8: TNLB_CUDA_TRY((launch_sell_col<Real, 8>(seg, cols, vals, x, y, alpha, beta, begin, end, win, st))); break;
                default: set_error("threads per segment must be 1, 2, 4 or 8 for column-major SlicedEllpack"); return TNLB_ERR_INVALID_ARGUMENT;
             }
          }
