@@ -17,6 +17,7 @@ from helpers import assert_spmv_close
 pytestmark = pytest.mark.gpu
 
 SHAPES = {  # rows, columns, half band (None: anywhere)
+    # clipped columns: the first and the last one are shared by thousands of rows
     "narrow": (310007, 310007, 400), "wide": (310007, 310007, 20000), "anywhere": (310007, 310007, None),
     "few_columns": (310007, 200003, 5000), "many_columns": (310007, 400009, 5000),
     "mixed": (310007, 310007, "mixed"),  # first half of the rows in a band, the others anywhere

@@ -74,9 +74,61 @@ __global__ void k_spmv_transposed(SegView v, const int32_t* __restrict__ cols, c
 // coalesced.  CSR rows are taken by G lanes, kScatterRows rows in flight; Col:
 // column-major Ellpack and SlicedEllpack, a lane a row, whose slots the lanes
 // read together.  A^T x of 13.5M entries at 500,009 rows in a band of 12,600
-// (FP64): 147 us with every addition in memory, 89 so.
+// (FP64): 147 us with every addition in memory, 79 so, 88 with all of the shared
+// memory as window: 163 KB leave the L1 cache enough for x and for the additions
+// outside.
+// A block first looks at some of its columns and adds all in memory where the
+// window does not pay (scatter_pays).
 constexpr int kScatterThreads = 1024, kScatterRows = 4;
+constexpr int kScatterBytes = 163 * 1024;
 extern __shared__ __align__(16) unsigned char scatter_smem[];
+
+// The column of one slot of a row among [r0, r1), or -1: of 32 neighbouring rows in
+// 8 places, one for each of the block's first 256 threads.
+template <bool Col>
+__device__ __forceinline__ int32_t scatter_sample(const SegView& v, const int32_t* __restrict__ cols, int32_t r0,
+                                                  int32_t r1)
+{
+   const int32_t r = r0 + (int32_t)((threadIdx.x >> 5) * (int64_t)(r1 - r0) / 8) + (int32_t)(threadIdx.x & 31);
+   if (threadIdx.x >= 256 || r >= r1) return -1;
+   const uint32_t any = threadIdx.x * 2654435761u >> 8;
+   if constexpr (Col) {
+      const bool sliced = v.format == TNLB_SLICED_ELLPACK;
+      const int32_t w = sliced ? v.slice_w[r / kSellSlice] : v.segment_size;
+      const int64_t base = sliced ? v.slice_off[r / kSellSlice] + (int64_t)(r % kSellSlice) : r;
+      return w > 0 ? cols[base + (int64_t)(any % (uint32_t)w) * (sliced ? kSellSlice : v.aligned_size)] : -1;
+   }
+   else {
+      const int32_t at = v.offsets[r], len = v.offsets[r + 1] - at;
+      return len > 0 ? cols[at + (int32_t)(any % (uint32_t)len)] : -1;
+   }
+}
+
+// Clears the window of `width` entries from `lo` and tells whether it pays for the
+// rows whose sampled columns the threads hold: an eighth of them lies in it, and
+// no column is kScatterHot of the 256.  Additions to one place in shared memory
+// follow one another, about 50 cycles each, which those to the L2 cache need not.
+// FP64, transposed, 27 entries a row at 500,009 rows, us by the kernels above, by
+// additions in memory here, and by the window: band of 40,000 150, 110, 93; of
+// 120,000 (17% inside) 149, 110, 95; random 148, 105, 103; a tenth of each 3000
+// rows' entries in one column 324, 128, 312; 63,000 entries in the first and the
+// last column 259, 144, 1123 (95 where only the blocks that hold them add in
+// memory).
+constexpr int kScatterHot = 5, kScatterBins = 8192;
+template <typename Real>
+__device__ __forceinline__ bool scatter_pays(int32_t c, int32_t lo, uint32_t width)
+{
+   int* words = reinterpret_cast<int*>(scatter_smem);
+   const uint32_t clear = max(width * (uint32_t)(sizeof(Real) / sizeof(int)), (uint32_t)kScatterBins);
+   for (uint32_t j = threadIdx.x; j < clear; j += kScatterThreads) words[j] = 0;
+   const int valid = __syncthreads_count(c >= 0);
+   const int inside = __syncthreads_count(c >= 0 && (uint32_t)(c - lo) < width);
+   int* bin = words + ((uint32_t)c * 2654435761u >> 19);
+   const bool hot = __syncthreads_or(c >= 0 && atomicAdd(bin, 1) >= kScatterHot - 1);
+   if (c >= 0) *bin = 0;
+   __syncthreads();
+   return 8 * inside >= valid && !hot;
+}
 
 template <typename Real, bool Symmetric, bool Col, int G>
 __global__ void __launch_bounds__(kScatterThreads, 1)
@@ -89,9 +141,8 @@ __global__ void __launch_bounds__(kScatterThreads, 1)
    const int32_t r1 = (int32_t)imin64((int64_t)r0 + per_block, row1);
    const int64_t mid = ((int64_t)r0 + r1) / 2;
    const int32_t lo = (int32_t)imin64(imax64(mid - room / 2, 0), imax64((int64_t)columns - room, 0));
-   const uint32_t width = (uint32_t)imin64(room, columns - lo);
-   for (uint32_t j = threadIdx.x; j < width; j += kScatterThreads) win[j] = Real(0);
-   __syncthreads();
+   uint32_t width = (uint32_t)imin64(room, columns - lo);
+   if (!scatter_pays<Real>(scatter_sample<Col>(v, cols, r0, r1), lo, width)) width = 0;
    auto add = [&](int32_t c, Real t) {
       const uint32_t at = (uint32_t)(c - lo);
       if (at < width)
@@ -194,8 +245,10 @@ int lanes_for(const tnlb_segments* seg)
 // the faster one (false: not launched).  Measured against the kernels above on
 // grids, band matrices (9 to 45 entries a row) and power-law rows:
 //  * column-major formats, whose slots those kernels read lane by lane: 1.3 to 3
-//    times as fast from 8000 entries an SM, 0.7 to 1.2 at 2600 to 4000;
-//  * transposed CSR: 1.1 to 2.1 times from 14,000 entries an SM, 0.9 at 10,000,
+//    times as fast from 8000 entries an SM, 0.7 to 1.2 at 2600 to 4000 (random
+//    columns, 4 to 42 a row, 0.95 to 2.1 from 8000);
+//  * transposed CSR: 1.1 to 2.1 times from 14,000 entries an SM (random columns
+//    1.1 to 1.8), 0.9 at 10,000,
 //    where the clearing and the flush of the window count; 0.3 to 0.7 on
 //    power-law rows, which one block's lanes cannot share, so rows are short;
 //  * symmetric CSR: 0.8 to 1.1, so never.
@@ -210,17 +263,16 @@ bool launch_scatter(const tnlb_segments* seg, const int32_t* cols, const Real* v
                     seg->max_row <= kScatterCsrRow;
    const bool col = (seg->format == TNLB_ELLPACK || seg->format == TNLB_SLICED_ELLPACK) &&
                     seg->organization == TNLB_COLUMN_MAJOR;
-   int dev = 0, sms = 0, smem = 0;
+   int dev = 0, sms = 0;
    if (!(csr || col) || cudaGetDevice(&dev) != cudaSuccess ||
-       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-       cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) {
+       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
       cudaGetLastError();
       return false;
    }
    const int64_t rows = (int64_t)row1 - row0;
    const int32_t per_block = (int32_t)((rows + sms - 1) / sms);
    if (seg->elements < (int64_t)sms * (col ? kScatterColEntries : kScatterCsrEntries) || per_block < 1) return false;
-   const int32_t room = (int32_t)(smem / sizeof(Real));
+   const int32_t room = (int32_t)(kScatterBytes / sizeof(Real));
    const int G = lanes_for(seg);
    auto* k = k_scatter_window<Real, Symmetric, true, 32>;
    if constexpr (!Symmetric)
@@ -229,11 +281,11 @@ bool launch_scatter(const tnlb_segments* seg, const int32_t* cols, const Real* v
              : G == 8  ? k_scatter_window<Real, false, false, 8>
              : G == 16 ? k_scatter_window<Real, false, false, 16>
                        : k_scatter_window<Real, false, false, 32>;
-   if (cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
+   if (cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, kScatterBytes) != cudaSuccess) {
       cudaGetLastError();
       return false;
    }
-   k<<<(unsigned)((rows + per_block - 1) / per_block), kScatterThreads, (size_t)room * sizeof(Real), st>>>(
+   k<<<(unsigned)((rows + per_block - 1) / per_block), kScatterThreads, kScatterBytes, st>>>(
       view_of(seg), cols, vals, x, y, alpha, row0, row1, per_block, columns, room, begin, end);
    *err = cudaGetLastError();
    return true;
