@@ -679,8 +679,14 @@ __global__ void __launch_bounds__(1024, 1)
 // kClusterRows rows one cluster, all of whose vectors (the owner's and the
 // `gathered` ones) have to fit shared memory.  `warp_stage`: bytes of a warp's
 // staged entries.
+// us an iteration of CG over the grid and in the cluster (FP64; BiCGStab and FP32
+// alike unless stated): 5 slots 3000 rows 8.1 and 3.3, 20,000 8.4 and 5.9, 40,000
+// 8.8 and 7.8; 7 slots 20,000 8.4 and 6.3, 40,000 8.9 and 8.6.  16 SMs read wide
+// rows too slowly: 15 slots 10,000 rows 8.7 and 7.4, 14,000 8.4 and 9.0, 20,000 8.7
+// and 10.8 (FP32 20,000 9.2 and 8.8).  30 GMRES steps (MGSR): 20,000 rows 3036 and
+// 2610, 60,000 3117 and 3103.
 constexpr int32_t kPersistMinRows = 128;
-constexpr int64_t kClusterRows = 20000;
+constexpr int64_t kClusterRows = 20000, kClusterWideRows = 12000;
 
 bool persist_shape(const void* kernel, bool cluster, int64_t n, int vectors, int gathered, size_t real, int warp_stage,
                    PersistShape& sh)
@@ -752,10 +758,11 @@ int64_t l2_bytes()
 
 // `pick(sync)`: the kernel for PersistGrid or PersistCluster.
 template <typename Pick>
-PersistShape persist_choose(Pick&& pick, int64_t n, int vectors, int gathered, size_t real, int warp_stage)
+PersistShape persist_choose(Pick&& pick, int64_t n, int vectors, int gathered, size_t real, int warp_stage,
+                            int64_t cluster_rows)
 {
    PersistShape sh;
-   if (n > kClusterRows || !persist_shape(pick(PersistCluster(PersistSync{})), true, n, vectors, gathered, real, 0, sh))
+   if (n > cluster_rows || !persist_shape(pick(PersistCluster(PersistSync{})), true, n, vectors, gathered, real, 0, sh))
       persist_shape(pick(PersistGrid(PersistSync{})), false, n, vectors, gathered, real, warp_stage, sh);
    return sh;
 }
@@ -775,6 +782,12 @@ int persist_stage(const tnlb_segments* seg)
    return seg->max_row <= 8 ? kPersistStage<Real, 8> : kPersistStage<Real, 16>;
 }
 
+template <typename Real>
+int64_t cluster_rows(const tnlb_segments* seg)
+{
+   return sizeof(Real) == 8 && persist_longest(seg) > 8 ? kClusterWideRows : kClusterRows;
+}
+
 }  // namespace
 
 template <typename Real>
@@ -782,7 +795,7 @@ PersistShape persist_cg(const tnlb_segments* seg)
 {
    if (!persist_pays(seg, sizeof(Real), false, l2_bytes())) return {};
    return persist_choose([&](auto sync) { return TNLB_PERSIST_FORMAT(k_cg_persist, Real, decltype(sync), seg); },
-                         seg->n, 4, 1, sizeof(Real), persist_stage<Real>(seg));
+                         seg->n, 4, 1, sizeof(Real), persist_stage<Real>(seg), cluster_rows<Real>(seg));
 }
 
 template <typename Real>
@@ -790,14 +803,14 @@ PersistShape persist_bicgstab(const tnlb_segments* seg)
 {
    if (!persist_pays(seg, sizeof(Real), true, l2_bytes())) return {};
    return persist_choose([&](auto sync) { return TNLB_PERSIST_FORMAT(k_bicg_persist, Real, decltype(sync), seg); },
-                         seg->n, 6, 2, sizeof(Real), persist_stage<Real>(seg));
+                         seg->n, 6, 2, sizeof(Real), persist_stage<Real>(seg), cluster_rows<Real>(seg));
 }
 
 template <typename Real>
 PersistShape persist_mgs(int64_t n)
 {
    PersistShape sh = persist_choose([&](auto sync) { return (const void*)k_mgs_persist<Real, decltype(sync)>; }, n, 3,
-                                    0, sizeof(Real), 0);
+                                    0, sizeof(Real), 0, kClusterRows);
    if (sh.kept < 3) sh.kernel = nullptr;
    return sh;
 }
