@@ -1,11 +1,14 @@
 """CG and BiCGStab in one resident kernel, against the same iterations in
 FP64 numpy.
 
-Sizes at the edges of the split over blocks: one row, a block's smallest run
-of 128 rows and one more, runs that are no multiple of 32, and more rows than
-the owners' vectors have room for in shared memory.  Well-conditioned
-matrices and a few iterations, so that rounding does not grow: one iteration
-adds a few ulp of the largest entries, 1e-13 and 2e-5 are over 50 times that.
+Sizes at the edges of the split over blocks, rows of 5, 8 and 16 slots at
+most in each.  Up to 20,000 rows (12,000 of more than 8 FP64 slots) one
+cluster of 16 blocks: one row, fewer rows than blocks have, a last block that
+is not full.  Above that the grid: the smallest, runs that are no multiple of
+32, every format and organisation, and more rows than the owners' vectors have
+room for in shared memory.  Well-conditioned matrices and a few iterations, so
+that rounding does not grow: one iteration adds a few ulp of the largest
+entries, 1e-13 and 2e-5 are over 50 times that.
 """
 import numpy as np
 import pytest
@@ -70,6 +73,10 @@ def _bicgstab(A, M, b, steps):
 
 CASES = [(1, (), "CSR", None), (128, (1,), "CSR", None), (129, (1, 5), "Ellpack", 0), (4001, (3, 70), "Ellpack", 1),
          (4001, (1, 2, 3, 70), "SlicedEllpack", 0), (19009, (1, 2, 3, 4, 5, 600), "SlicedEllpack", 1),
+         (12001, (1, 2, 3, 4, 5, 6, 90), "CSR", None), (20001, (1, 40), "SlicedEllpack", 1),
+         (20011, (1, 2, 3, 4, 5, 6, 300), "CSR", None), (40009, (2, 70), "Ellpack", 0),
+         (40009, (1, 2, 70), "Ellpack", 1), (40009, (1, 2, 3, 4, 5, 70), "SlicedEllpack", 0),
+         (40009, (1, 2, 3, 4, 5, 70), "SlicedEllpack", 1), (90001, (1, 2, 3, 4, 5, 600), "Ellpack", 1),
          (151553, (1, 2, 300), "CSR", None), (1500007, (1, 1200), "CSR", None)]
 
 
@@ -109,12 +116,12 @@ def test_resident_solver_matches_numpy(n, offsets, fmt, org, solver, precond, re
         assert err <= (1e-13 if real == "float64" else 2e-5) * np.linalg.norm(want)
 
 
-def test_resident_bicgstab_restarts():
+@pytest.mark.parametrize("n", [4001, 40009])  # one cluster, the grid
+def test_resident_bicgstab_restarts(n):
     """100 iterations where 30 reach the rounding level: (r, r_ast) falls below
     the restart's threshold again and again, and x stays the solution."""
     import tnl_b200 as t
 
-    n = 4001
     rp, cols, vals, rows = _matrix(n, (1, 70), False, 7)
     want = np.random.default_rng(2).uniform(-1, 1, n)
     b = np.bincount(rows, vals * want[cols], minlength=n)
@@ -185,3 +192,44 @@ def test_resident_gram_schmidt_matches_numpy(n, variant, real):
     S.solve(torch.tensor(b, dtype=dtype, device="cuda"), y)
     err = np.linalg.norm(y.cpu().numpy().astype(np.float64) - x)
     assert err <= (1e-13 if real == "float64" else 2e-5) * np.linalg.norm(x)
+
+
+def test_resident_solvers_on_two_streams():
+    """Two threads, each on a stream of its own, with systems of different forms:
+    the results of one thread alone."""
+    import threading
+
+    import tnl_b200 as t
+
+    systems = []
+    for k, (n, offsets, solver) in enumerate([(9001, (1, 70), "CG"), (60013, (1, 2, 300), "BICGStab"),
+                                              (60013, (1, 300), "CG"), (9001, (1, 2, 70), "GMRES")]):
+        rp, cols, vals, _ = _matrix(n, offsets, solver == "CG", k)
+        mat = t.SparseMatrix(t.CSR, torch.float64).assign(rp, cols, vals)
+        systems.append((solver, mat, torch.tensor(np.random.default_rng(k).uniform(-1, 1, n), device="cuda")))
+    torch.cuda.synchronize()
+
+    def solve(which, out):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for solver, mat, b in which:
+                S = getattr(t, solver)()
+                S.setMatrix(mat)
+                S.setConvergenceResidue(0.0)
+                S.setMaxIterations(ITERATIONS)
+                x = torch.zeros_like(b)
+                S.solve(b, x)
+                out.append(x)
+
+    want = []
+    solve(systems, want)
+    for _ in range(3):
+        got = [[], []]
+        threads = [threading.Thread(target=solve, args=(order, out))
+                   for order, out in ((systems, got[0]), (systems[::-1], got[1]))]
+        for th in threads:
+            th.start()
+        for th in threads:
+            th.join()
+        assert len(got[0]) == len(got[1]) == len(want)
+        for a, b, w in zip(got[0], got[1][::-1], want):
+            assert torch.equal(a, w) and torch.equal(b, w)
