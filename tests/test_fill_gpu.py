@@ -38,3 +38,21 @@ def test_fill_writes_every_slot(n, fmt, org, real):
         at = seg.getGlobalIndex(r, local)
         want_c[at], want_v[at] = cols[keep], vals[keep]
         assert np.array_equal(c, want_c) and np.array_equal(v, want_v)
+
+
+def test_failed_fill_leaves_padding(monkeypatch):
+    """A fill that fails leaves a matrix without elements, whatever the memory
+    held before."""
+    import tnl_b200 as t
+
+    rp = np.arange(0, 3 * 1001, 3, dtype=np.int32)
+    cols, vals = np.tile(np.arange(3, dtype=np.int32), 1000), np.ones(3000)
+    held = [torch.full((3072,), 7, dtype=torch.int32, device="cuda") for _ in range(8)]
+    held += [torch.full((3072,), 7.0, dtype=torch.float64, device="cuda") for _ in range(8)]
+    del held
+    M = t.SparseMatrix(t.SlicedEllpack, torch.float64)
+    monkeypatch.setattr(t.capi, "tnlb_matrix_fill_from_csr", lambda *a: t.capi.ERR_INVALID_ARGUMENT)
+    with pytest.raises(ValueError):
+        M.assign(rp, cols, vals, 3)
+    assert M.getColumnIndexes().numel() == 3072
+    assert (M.getColumnIndexes() == -1).all() and (M.getValues() == 0).all()

@@ -303,10 +303,15 @@ class SparseMatrix:
         v = v.to(device="cuda", dtype=self.real).contiguous()
         self.setDimensions(n, n if columns is None else columns)
         self._allocate(rp[1:] - rp[:-1])  # the fill writes every slot
-        check(capi.tnlb_matrix_fill_from_csr(self.segments.handle, _real_code(self.real), rp.data_ptr(),
-                                             c.data_ptr() if c.numel() else None, v.data_ptr() if v.numel() else None,
-                                             self.columnIndexes.data_ptr() if self.columnIndexes.numel() else None,
-                                             self.values.data_ptr() if self.values.numel() else None, _stream()))
+        status = capi.tnlb_matrix_fill_from_csr(
+            self.segments.handle, _real_code(self.real), rp.data_ptr(), c.data_ptr() if c.numel() else None,
+            v.data_ptr() if v.numel() else None,
+            self.columnIndexes.data_ptr() if self.columnIndexes.numel() else None,
+            self.values.data_ptr() if self.values.numel() else None, _stream())
+        if status != capi.OK:  # no column may be left that a product would gather from
+            self.values.zero_()
+            self.columnIndexes.fill_(-1)
+        check(status)
         return self
 
     @classmethod
