@@ -137,3 +137,37 @@ def test_pipelined_ilu0_apply_fp32():
     xs = torch.empty(A.n, dtype=torch.float32, device="cuda")
     P.solve(torch.tensor(b, device="cuda"), xs)
     assert np.array_equal(xs.cpu().numpy(), x)
+
+
+@pytest.mark.parametrize("side", [40, 300])  # level by level or one part, several parts
+def test_ilu0_applied_from_two_threads(oracle, side):
+    """One preconditioner on two streams at once: each application as if alone."""
+    import threading
+
+    import tnl_b200 as t
+    from tnl_b200 import generators as g
+
+    A = _coupled(0, side)
+    M = t.SparseMatrix(t.CSR, torch.float64).assign(A.rowptr, A.cols, A.vals)
+    P = t.ILU0()
+    P.update(M)
+    b = [g.uniform_vector(A.n, seed) for seed in (3, 4)]
+    bs = [torch.tensor(v, device="cuda") for v in b]
+    torch.cuda.synchronize()
+    out = [[], []]
+
+    def run(k):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(20):
+                x = torch.empty_like(bs[k])
+                P.solve(bs[k], x)
+                out[k].append(x)
+
+    threads = [threading.Thread(target=run, args=(k,)) for k in (0, 1)]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    for k in (0, 1):
+        want = oracle.prec_apply(A, 2, b[k])
+        assert len(out[k]) == 20 and all(np.array_equal(x.cpu().numpy(), want) for x in out[k])

@@ -18,6 +18,7 @@
 // column order, unit-diagonal L), with separately rounded multiply and
 // subtract, so the factors and the solves are bit-identical to the Host.
 #include <algorithm>
+#include <mutex>
 #include <vector>
 
 #include "ilu_pipe.cuh"
@@ -402,6 +403,8 @@ struct Ilu0 : Ilu0Base {
    bool pipe = false;  // whether the solves run as pipelines (ilu_pipe.cuh)
    PipeTri<Real> lpipe, upipe;
    DeviceBuffer lin, uin, progress;
+   std::mutex order;
+   cudaEvent_t done = nullptr;  // the last application
    int32_t* pipe_failed = nullptr;  // host memory that the pipeline's kernels write when a wait runs out
    std::vector<int32_t> lptr, uptr;  // level boundaries into lrows / urows
    cudaGraphExec_t exec = nullptr;
@@ -413,6 +416,7 @@ struct Ilu0 : Ilu0Base {
    {
       if (exec) cudaGraphExecDestroy(exec);
       if (cs) cudaStreamDestroy(cs);
+      if (done) cudaEventDestroy(done);
       if (pipe_failed) cudaFreeHost(pipe_failed);
    }
 
@@ -542,11 +546,24 @@ struct Ilu0 : Ilu0Base {
       return TNLB_ERR_CUDA;
    }
 
+   // One application after the other, whichever streams and threads they come from:
+   // they share the object's buffers, and the pipeline's progress words.
    tnlb_status apply(const void* bv, void* xv, cudaStream_t st) override
    {
       const Real* b = static_cast<const Real*>(bv);
       Real* x = static_cast<Real*>(xv);
-      if (pipe) return apply_pipe(b, x, st);
+      std::lock_guard<std::mutex> lock(order);
+      if (done)
+         TNLB_CUDA_TRY(cudaStreamWaitEvent(st, done, 0));
+      else
+         TNLB_CUDA_TRY(cudaEventCreateWithFlags(&done, cudaEventDisableTiming));
+      TNLB_TRY_STATUS(pipe ? apply_pipe(b, x, st) : apply_levels(b, x, st));
+      TNLB_CUDA_TRY(cudaEventRecord(done, st));
+      return TNLB_OK;
+   }
+
+   tnlb_status apply_levels(const Real* b, Real* x, cudaStream_t st)
+   {
       // Solves are replayed from a graph captured for fixed (b, x) buffers:
       // copy in/out of the graph's own buffers when the caller's differ.
       if (!exec) {
