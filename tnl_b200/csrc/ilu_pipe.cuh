@@ -572,8 +572,9 @@ __global__ void __launch_bounds__((kPipeMaxStages + 3) * 32 + kPipeStepRows, 1) 
          __syncwarp();
          filled ^= 1u;
       }
-      // the last copies have landed before the block ends, also where nobody waited for them
-      if (lane == 0 && s < count) pipe_bar_wait(&s_full[s], filled, patience);
+      // the last copies have landed before the block ends, also where nobody waited for
+      // them and a failure ends the other waits
+      if (lane == 0 && s < count) band_wait(&s_full[s], filled);
    }
    __syncthreads();
    if (*const_cast<volatile int32_t*>(&s_failed))
